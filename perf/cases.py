@@ -286,6 +286,13 @@ def prepare(case, seed):
             "p": pinned_like(flow.p).copy_(flow.p), "bulk": torch.zeros(2, dtype=torch.float64).pin_memory()}
 
 
+def _bulk(c, both):
+    """[u_bulk, forcing] pairs.  The forcing is the bulk velocity's tiny
+    defect over dt: in the mixed form it is the sum of the FP32 rounding of a
+    step, which has no value to compare, so only the bulk velocity is given."""
+    return both if c["precision"] == "fp64" else both.view(-1, 2)[:, 0]
+
+
 def run(state):
     c = state["c"]
     if c["kind"] == "step":
@@ -296,7 +303,8 @@ def run(state):
             state["done"] = 0
         state["done"] += 1
         bulk, forcing = flow.step_sl_bdf2(c["dt"])
-        return {"u": flow.u, "v": flow.v, "w": flow.w, "p": flow.p, "bulk": bulk, "forcing": forcing}
+        return {"V": (flow.u, flow.v, flow.w), "p": flow.p,
+                "bulk": (bulk, forcing) if c["precision"] == "fp64" else bulk}
     if c["kind"] == "advect":
         adv, extra = state["adv"], state["extra"]
         out = adv.advect(*state["f"], *state["mid"], c["dt"], extra_rhs=extra if extra else None)
@@ -310,7 +318,7 @@ def run(state):
             state["done"] = 0
         state["done"] += 1
         ens.step()
-        return {"V": [ens.velocity(i) for i in range(ens.n)], "p": ens.p, "bulk": ens.bulk_out}
+        return {"V": [ens.velocity(i) for i in range(ens.n)], "p": ens.p, "bulk": _bulk(c, ens.bulk_out)}
     if c["kind"] == "gradient":
         V0 = [t.detach().requires_grad_(True) for t in state["V0"]]
         VN = SLRollout.apply(*V0, state["flow"], c["dt"], c["steps"], c["every"])
@@ -322,7 +330,7 @@ def run(state):
     level = lambda i: state["first"][i + 2] if i < 0 else state["ring"][i % 3]  # noqa: E731
     prev, cur, nxt = level(k - 2), level(k - 1), level(k)
     state["stepper"].step(cur, prev, nxt, state["p"], state["bulk"], c["dt"])
-    return {"V": nxt, "p": state["p"], "bulk": state["bulk"]}
+    return {"V": nxt, "p": state["p"], "bulk": _bulk(c, state["bulk"])}
 
 
 def work(case):
@@ -565,14 +573,15 @@ def exact(case, seed):
     c = _full(case)
     if c["kind"] == "ensemble":
         got = [_Plain(m).two_steps(seed) for m in _members(c)]
-        return {"V": [g[0] for g in got], "p": [g[1] for g in got], "bulk": torch.cat([g[2] for g in got])}
+        return {"V": [g[0] for g in got], "p": [g[1] for g in got],
+                "bulk": _bulk(c, torch.cat([g[2] for g in got]))}
     plain = _Plain(c)
     if c["kind"] == "step":
-        (u, v, w), p, b = plain.two_steps(seed)
-        return {"u": u, "v": v, "w": w, "p": p, "bulk": b[0], "forcing": b[1]}
+        V, p, b = plain.two_steps(seed)
+        return {"V": V, "p": p, "bulk": (b[0], b[1]) if c["precision"] == "fp64" else b[0]}
     if c["kind"] == "host":
         V, p, b = plain.two_steps(seed)
-        return {"V": V, "p": p, "bulk": b}
+        return {"V": V, "p": p, "bulk": _bulk(c, b)}
     if c["kind"] == "advect":
         # what lies outside the interiors of the advector's buffers is not refreshed
         triples, mid = _advect_inputs(c, seed)
