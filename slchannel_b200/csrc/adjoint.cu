@@ -135,13 +135,13 @@ __device__ __forceinline__ GBase<C, O> gather_base(const SlcParams &P, double x,
     double s = x * P.inv_dx + Comp<C>::shift_x;
     double f = floor(s);
     g.tx = s - f;
-    g.bx0 = wrapn(wrap_base(f, P.nx) - h, P.nx);
+    g.bx0 = wrapn(wrap_base(f, P.nx, P.inv_nx) - h, P.nx);
     s = y * P.inv_dy + Comp<C>::shift_y;
     f = floor(s);
     g.ty = s - f;
-    g.by0 = wrapn(wrap_base(f, P.ny) - h, P.ny);
+    g.by0 = wrapn(wrap_base(f, P.ny, P.inv_ny) - h, P.ny);
     const int NZ = Comp<C>::centers ? P.nz + 2 : P.nz + 1;
-    const int m0 = locate_m0(P, Comp<C>::centers, face_cell(P, z), z);
+    const int m0 = locate_m0(Comp<C>::centers, half_cell(P, z));
     g.k0 = min(max(m0 - h, 0), NZ - O);
     return g;
 }
@@ -244,7 +244,7 @@ __device__ __forceinline__ void sample3_grad(const SlcParams &P, const V3 &M, do
 {
     const double zc = clampz(P, z);
     TriShared t;
-    tri_shared(P, x, y, zc, face_cell(P, zc), t);
+    tri_shared(P, x, y, zc, half_cell(P, zc), t);
     const NodeView<double> F[3] = {M.u, M.v, M.w};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -442,7 +442,7 @@ __global__ void k_tri_keys(SlcParams P, int c, const TriRec *__restrict__ tri, l
     const TriRec R = tri[r];
     const double zc = clampz(P, R.z);
     TriShared t;
-    tri_shared(P, R.x, R.y, zc, face_cell(P, zc), t);
+    tri_shared(P, R.x, R.y, zc, half_cell(P, zc), t);
     const TriPiece q = tri_piece(P, c, t);
     const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
     keys[r] = (q.i0 * P.ny + q.j0) * NZ + q.k0;

@@ -459,7 +459,7 @@ __device__ __forceinline__ void bulk_finish(const double *__restrict__ partials,
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        const double bulk = red[0] * dxdy_over_V;
+        const double bulk = __dmul_rn(red[0], dxdy_over_V);  // not fused into U_bulk - bulk: alike in every kernel
         if (bulk_out) *bulk_out = bulk;
         if (shift_out) {
             const double corr = U_bulk - bulk;

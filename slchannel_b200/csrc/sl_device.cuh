@@ -20,7 +20,7 @@ __device__ __forceinline__ void sample3(const SlcParams &P, const Vel3 &M, doubl
 {
     const double zc = clampz(P, z);
     TriShared t;
-    tri_shared(P, x, y, zc, face_cell(P, zc), t);
+    tri_shared(P, x, y, zc, half_cell(P, zc), t);
     us = tri_sample(M.u, t.ia0, t.ia1, t.txa, t.jb0, t.jb1, t.tyb, t.kc, t.wc0, t.wc1);
     vs = tri_sample(M.v, t.ib0, t.ib1, t.txb, t.ja0, t.ja1, t.tya, t.kc, t.wc0, t.wc1);
     ws = tri_sample(M.w, t.ib0, t.ib1, t.txb, t.jb0, t.jb1, t.tyb, t.kf, t.wf0, t.wf1);
@@ -34,7 +34,7 @@ __device__ __noinline__ void sample3_o4(const SlcParams &P, const Vel3 &M, doubl
                                         double z, double &us, double &vs, double &ws)
 {
     const double zc = clampz(P, z);
-    const int c = face_cell(P, zc);
+    const int c = half_cell(P, zc);
     Stencil<4, double> st;
     build_stencil<0, 4, double>(P, M.u.sx, M.u.sy, x, y, zc, c, st);
     us = gather_sum<4, double, double>(M.u.p, st);
@@ -65,21 +65,23 @@ __device__ __forceinline__ void first_sample(const SlcParams &P, const Vel3 &M, 
 
 // Iterated midpoint rule continued from the first-iteration sample
 // (us0, vs0, ws0) taken at the arrival point; returns the unclamped foot.
-template <int TO = 0>
+// NI: the number of iterations at compile time (no loop, so that the samples
+// of several feet can be in flight together), 0 to read P.n_iters.
+template <int TO = 0, int NI = 0>
 __device__ __forceinline__ void trace_foot(const SlcParams &P, const Vel3 &M, double xa, double ya,
                                            double za, double half_dt, double us0, double vs0,
                                            double ws0, double &xd, double &yd, double &zd)
 {
-    double xm = xa - half_dt * us0;
-    double ym = ya - half_dt * vs0;
-    double zm = clampz(P, za - half_dt * ws0);
-    for (int it = 1; it < P.n_iters; ++it) {
+    double xm = fma(-half_dt, us0, xa);
+    double ym = fma(-half_dt, vs0, ya);
+    double zm = clampz(P, fma(-half_dt, ws0, za));
+    for (int it = 1; it < (NI ? NI : P.n_iters); ++it) {
         double us, vs, ws;
         if (traj4<TO>(P)) sample3_o4(P, M, xm, ym, zm, us, vs, ws);
         else sample3(P, M, xm, ym, zm, us, vs, ws);
-        xm = xa - half_dt * us;
-        ym = ya - half_dt * vs;
-        zm = clampz(P, za - half_dt * ws);
+        xm = fma(-half_dt, us, xa);
+        ym = fma(-half_dt, vs, ya);
+        zm = clampz(P, fma(-half_dt, ws, za));
     }
     xd = 2.0 * xm - xa;
     yd = 2.0 * ym - ya;
@@ -93,7 +95,7 @@ __device__ __forceinline__ double gather_foot(const SlcParams &P, NodeView<doubl
 {
     if (zd < P.z_lo || zd > P.z_hi) ncl += 1;
     double z = clampz(P, zd);
-    int c = face_cell(P, z);
+    const int c = half_cell(P, z);
     Stencil<O, double> st;
     build_stencil<C, O, double>(P, F.sx, F.sy, xd, yd, z, c, st);
     return gather_sum<O, double, double>(F.p, st);
@@ -113,10 +115,24 @@ __device__ __forceinline__ double xy_diffusion(const SlcParams &P, const double 
     if (C == 0 && Ip == P.nx + 1) Ip = 1;
     if (C == 1 && Jp == P.ny + 1) Jp = 1;
     const double fc = __ldg(f + I * sx + J * sy + K);
-    const double d2x =
-        (__ldg(f + Ip * sx + J * sy + K) - 2.0 * fc + __ldg(f + (I - 1) * sx + J * sy + K)) * P.inv_dx2;
-    const double d2y =
-        (__ldg(f + I * sx + Jp * sy + K) - 2.0 * fc + __ldg(f + I * sx + (J - 1) * sy + K)) * P.inv_dy2;
-    return P.nu * (d2x + d2y);
+    const double d2x = fma(-2.0, fc, __ldg(f + Ip * sx + J * sy + K)) + __ldg(f + (I - 1) * sx + J * sy + K);
+    const double d2y = fma(-2.0, fc, __ldg(f + I * sx + Jp * sy + K)) + __ldg(f + I * sx + (J - 1) * sy + K);
+    return __dmul_rn(P.nu, dot2(d2x, P.inv_dx2, d2y, P.inv_dy2));
+}
+
+// The explicit x, y diffusion of the BDF2 predictor: 2 R^n - R^{n-1}, or R^n
+// lagged (solver.py:846-903).
+template <int C>
+__device__ __forceinline__ double xy_diffusion_bdf2(const SlcParams &P, const double *__restrict__ fn,
+                                                    const double *__restrict__ fnm1, int i, int j, int k)
+{
+    const double Rn = xy_diffusion<C>(P, fn, i, j, k);
+    return P.xy_lagged ? Rn : fma(2.0, Rn, -xy_diffusion<C>(P, fnm1, i, j, k));
+}
+
+// 4/3 ubar - 1/3 ubarbar + (2/3) dt Rh (solver.py:846-903).
+__device__ __forceinline__ double bdf2_combine(double ubar, double ubb, double dt, double Rh)
+{
+    return fma((2.0 / 3.0) * dt, Rh, dot2(ubar, 4.0 / 3.0, ubb, -1.0 / 3.0));
 }
 

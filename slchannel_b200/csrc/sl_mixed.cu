@@ -37,11 +37,11 @@ struct Vel3M {
     MixedView u, v, w;
 };
 
-__device__ __forceinline__ void add_clamps(unsigned long long *counter, unsigned cnt)
-{
-    unsigned tot = __reduce_add_sync(0xffffffffu, cnt);
-    if ((threadIdx.x & 31) == 0 && tot) atomicAdd(counter, (unsigned long long)tot);
-}
+#include "sl_device.cuh"
+
+// a b + c d with the first product rounded (the FP32 arithmetic is written
+// with explicit roundings like the FP64 one, see dot2).
+__device__ __forceinline__ float dot2f(float a, float b, float c, float d) { return fmaf(c, d, __fmul_rn(a, b)); }
 
 // ---- FP32 characteristic trace -------------------------------------------
 // A trajectory point is its arrival point plus an FP32 displacement.  In
@@ -102,24 +102,6 @@ __device__ __forceinline__ float clampdz(const Arr32 &A, float dz)
     return dz < A.dzlo ? A.dzlo : (dz > A.dzhi ? A.dzhi : dz);
 }
 
-// FP32 face cell (analytic inverse tanh map, semilag.py:400-416).
-__device__ __forceinline__ int face_cell32(const SlcParams &P, float z)
-{
-    const float lim = 0.99999994f;
-    float kf;
-    if (P.symmetric) {
-        float arg = (z * (float)P.two_over_Lz - 1.0f) * (float)P.tanh_g;
-        arg = fminf(fmaxf(arg, -lim), lim);
-        kf = (atanhf(arg) * (float)P.inv_gamma + 1.0f) * (float)P.half_nz;
-    } else {
-        float arg = (1.0f - z * (float)P.inv_Lz) * (float)P.tanh_g;
-        arg = fminf(fmaxf(arg, -lim), lim);
-        kf = (1.0f - atanhf(arg) * (float)P.inv_gamma) * (float)P.nzd;
-    }
-    kf = fminf(fmaxf(floorf(kf), 0.0f), (float)(P.nz - 1));
-    return (int)kf;
-}
-
 __device__ __forceinline__ float tri32(MixedView V, int i0, int i1, float tx, int j0, int j1,
                                        float ty, int k0, float wz0, float wz1)
 {
@@ -128,12 +110,12 @@ __device__ __forceinline__ float tri32(MixedView V, int i0, int i1, float tx, in
     const float *p01 = F.p + i0 * F.sx + j1 * F.sy + k0;
     const float *p10 = F.p + i1 * F.sx + j0 * F.sy + k0;
     const float *p11 = F.p + i1 * F.sx + j1 * F.sy + k0;
-    const float a00 = wz0 * __ldg(p00) + wz1 * __ldg(p00 + 1);
-    const float a01 = wz0 * __ldg(p01) + wz1 * __ldg(p01 + 1);
-    const float a10 = wz0 * __ldg(p10) + wz1 * __ldg(p10 + 1);
-    const float a11 = wz0 * __ldg(p11) + wz1 * __ldg(p11 + 1);
-    const float fl = (1.f - tx) * ((1.f - ty) * a00 + ty * a01) + tx * ((1.f - ty) * a10 + ty * a11);
-    return fl + (wz0 * __ldg(V.mean32 + k0) + wz1 * __ldg(V.mean32 + k0 + 1));
+    const float a00 = dot2f(wz0, __ldg(p00), wz1, __ldg(p00 + 1));
+    const float a01 = dot2f(wz0, __ldg(p01), wz1, __ldg(p01 + 1));
+    const float a10 = dot2f(wz0, __ldg(p10), wz1, __ldg(p10 + 1));
+    const float a11 = dot2f(wz0, __ldg(p11), wz1, __ldg(p11 + 1));
+    const float fl = dot2f(1.f - tx, dot2f(1.f - ty, a00, ty, a01), tx, dot2f(1.f - ty, a10, ty, a11));
+    return fl + dot2f(wz0, __ldg(V.mean32 + k0), wz1, __ldg(V.mean32 + k0 + 1));
 }
 
 // Trajectory velocity at arrival + (ddx, ddy) (index units) and height
@@ -153,15 +135,11 @@ __device__ __forceinline__ void sample3_32(const SlcParams &P, const Vel3M &M, c
     const int ia1 = (ia0 + 1 == P.nx) ? 0 : ia0 + 1, ib1 = (ib0 + 1 == P.nx) ? 0 : ib0 + 1;
     const int ja1 = (ja0 + 1 == P.ny) ? 0 : ja0 + 1, jb1 = (jb0 + 1 == P.ny) ? 0 : jb0 + 1;
     const double z = A.za + (double)dz;
-    const int c = face_cell32(P, (float)z);
-    const int kc = min(max(c + (z >= __ldg(P.zc + c + 1) ? 1 : 0), 0), P.nz);
-    const int kf = min(max(c, 0), P.nz - 1);
-    const float *dc = P.dinv_c32[2] + kc;  // order-2 tables: nz+1 / nz rows
-    const float *df = P.dinv_f32[2] + kf;
-    const float wc0 = (float)(z - __ldg(P.zc + kc + 1)) * __ldg(dc);
-    const float wc1 = (float)(z - __ldg(P.zc + kc)) * __ldg(dc + P.nz + 1);
-    const float wf0 = (float)(z - __ldg(P.zf + kf + 1)) * __ldg(df);
-    const float wf1 = (float)(z - __ldg(P.zf + kf)) * __ldg(df + P.nz);
+    const int half = half_cell(P, z);
+    const int kc = locate_m0(true, half), kf = locate_m0(false, half);
+    const double2 lc = __ldg(P.lin_c + kc), lf = __ldg(P.lin_f + kf);
+    const float wc1 = (float)((z - lc.x) * lc.y), wc0 = 1.f - wc1;
+    const float wf1 = (float)((z - lf.x) * lf.y), wf0 = 1.f - wf1;
     us = tri32(M.u, ia0, ia1, txa, jb0, jb1, tyb, kc, wc0, wc1);
     vs = tri32(M.v, ib0, ib1, txb, ja0, ja1, tya, kc, wc0, wc1);
     ws = tri32(M.w, ib0, ib1, txb, jb0, jb1, tyb, kf, wf0, wf1);
@@ -181,16 +159,16 @@ __device__ __forceinline__ void trace_foot32(const SlcParams &P, const Vel3M &M,
                                              float &ddx, float &ddy, float &ddz)
 {
     const float idx = (float)P.inv_dx, idy = (float)P.inv_dy;
-    float mx = -hdt * us0 * idx;
-    float my = -hdt * vs0 * idy;
-    float mz = clampdz(A, -hdt * ws0);
+    float mx = __fmul_rn(__fmul_rn(-hdt, us0), idx);
+    float my = __fmul_rn(__fmul_rn(-hdt, vs0), idy);
+    float mz = clampdz(A, __fmul_rn(-hdt, ws0));
     for (int it = 1; it < P.n_iters; ++it) {
         float us, vs, ws;
         if (TO == 4 || (TO == 0 && P.traj_order == 4)) sample3_32_o4(P, M, A, mx, my, mz, us, vs, ws);
         else sample3_32(P, M, A, mx, my, mz, us, vs, ws);
-        mx = -hdt * us * idx;
-        my = -hdt * vs * idy;
-        mz = clampdz(A, -hdt * ws);
+        mx = __fmul_rn(__fmul_rn(-hdt, us), idx);
+        my = __fmul_rn(__fmul_rn(-hdt, vs), idy);
+        mz = clampdz(A, __fmul_rn(-hdt, ws));
     }
     ddx = 2.f * mx;
     ddy = 2.f * my;
@@ -224,8 +202,7 @@ __device__ __forceinline__ double gather_foot32(const SlcParams &P, MixedView F,
     for (int m = 0; m < O; ++m) st.yoff[m] = wrap_index(by + m - h, P.ny) * F.f.sy;
     uniform_weights<O, float>(P, tx, st.wx);
     uniform_weights<O, float>(P, ty, st.wy);
-    const int c = face_cell32(P, (float)z);
-    const int m0 = Comp<C>::centers ? c + (z >= __ldg(P.zc + c + 1) ? 1 : 0) : c;
+    const int m0 = locate_m0(Comp<C>::centers, half_cell(P, z));
     const int k0 = min(max(m0 - h, 0), NZ - O);
     st.k0 = k0;
     // z - z_node from the FP64 node table: FP32-rounded nodes would break
@@ -296,24 +273,6 @@ struct NodeValMixed32 {
     }
 };
 
-template <int C>
-__device__ __forceinline__ double xy_diffusion64(const SlcParams &P, const double *__restrict__ f,
-                                                 int i, int j, int k)
-{
-    const GhostShape g = ghost_shape(C, P.nx, P.ny, P.nz);
-    const size_t sx = (size_t)g.Y * g.Z, sy = g.Z;
-    const int I = i + 1, J = j + 1, K = k + 1;
-    int Ip = I + 1, Jp = J + 1;
-    if (C == 0 && Ip == P.nx + 1) Ip = 1;
-    if (C == 1 && Jp == P.ny + 1) Jp = 1;
-    const double fc = __ldg(f + I * sx + J * sy + K);
-    const double d2x =
-        (__ldg(f + Ip * sx + J * sy + K) - 2.0 * fc + __ldg(f + (I - 1) * sx + J * sy + K)) * P.inv_dx2;
-    const double d2y =
-        (__ldg(f + I * sx + Jp * sy + K) - 2.0 * fc + __ldg(f + I * sx + (J - 1) * sy + K)) * P.inv_dy2;
-    return P.nu * (d2x + d2y);
-}
-
 // MODE 0: one foot of A (advect); 1: BDF1 predictor; 2: BDF2 predictor.
 // FA/FB: the mixed views of the near (V^n) and far (V^{n-1}) fields of
 // component C; fn/fnm1: the same fields in FP64 (ghost-shaped) for R.
@@ -353,7 +312,7 @@ __device__ __forceinline__ void sl_point_mixed(const SlcParams &P, const Vel3M &
         if (MODE == 0) {
             res = ubar;
         } else if (MODE == 1) {
-            res = ubar + dt * xy_diffusion64<C>(P, fn, i, j, k);
+            res = fma(dt, xy_diffusion<C>(P, fn, i, j, k), ubar);
         } else {
             if (FAR_FIRST) {
                 ddx = fdx;
@@ -363,10 +322,7 @@ __device__ __forceinline__ void sl_point_mixed(const SlcParams &P, const Vel3M &
                 trace_foot32<TO>(P, M, A, (float)dt, us0, vs0, ws0, ddx, ddy, ddz);
             }
             const double ubb = gather_foot32<C, O>(P, FB, A, ddx, ddy, ddz, ncl);
-            const double Rn = xy_diffusion64<C>(P, fn, i, j, k);
-            const double Rh = P.xy_lagged ? Rn : 2.0 * Rn - xy_diffusion64<C>(P, fnm1, i, j, k);
-            res = ubar * (4.0 / 3.0) + ubb * (-1.0 / 3.0);
-            res = res + ((2.0 / 3.0) * dt) * Rh;
+            res = bdf2_combine(ubar, ubb, dt, xy_diffusion_bdf2<C>(P, fn, fnm1, i, j, k));
         }
         if (MODE == 0 && om.sx != 0) {
             out[om.off + (long long)i * om.sx + (long long)j * om.sy + k] = res;
@@ -476,8 +432,7 @@ __device__ __forceinline__ FootM32 locate_foot_m32(const SlcParams &P, const Arr
     fl = floorf(fr);
     F.ty = fr - fl;
     F.ry = yi + (int)fl - h - j0;
-    const int c = face_cell32(P, (float)F.z);
-    const int m0 = Comp<C>::centers ? c + (F.z >= __ldg(P.zc + c + 1) ? 1 : 0) : c;
+    const int m0 = locate_m0(Comp<C>::centers, half_cell(P, F.z));
     F.k0 = min(max(m0 - h, 0), NZ - O);
     return F;
 }
@@ -685,10 +640,7 @@ __global__ void __launch_bounds__(kThreads, SLC_SLMT_MIN_BLOCKS)
             ubb = gather_box_m32<C, O>(P, FB, box, F, F.rx - red[6], F.ry - red[8], F.k0 - Z0);
         else
             ubb = gather_foot32<C, O>(P, FB, A, dx, dy, dz, none);
-        const double Rn = xy_diffusion64<C>(P, fn, i, j, k);
-        const double Rh = P.xy_lagged ? Rn : 2.0 * Rn - xy_diffusion64<C>(P, fnm1, i, j, k);
-        double res = ubar * (4.0 / 3.0) + ubb * (-1.0 / 3.0);
-        res = res + ((2.0 / 3.0) * dt) * Rh;
+        const double res = bdf2_combine(ubar, ubb, dt, xy_diffusion_bdf2<C>(P, fn, fnm1, i, j, k));
         const GhostShape g = ghost_shape(C, P.nx, P.ny, P.nz);
         out[(size_t)(i + 1) * g.Y * g.Z + (size_t)(j + 1) * g.Z + (k + 1)] = res;
     }

@@ -94,16 +94,16 @@ __device__ __forceinline__ Foot locate_foot(const SlcParams &P, double xd, doubl
     if (zd < P.z_lo || zd > P.z_hi) ncl += 1;
     Foot F;
     F.z = clampz(P, zd);
-    double s = xd * P.inv_dx + Comp<C>::shift_x;
+    double s = fma(xd, P.inv_dx, Comp<C>::shift_x);
     double f = floor(s);
     F.tx = s - f;
     F.rx = rel_base(f, h, i0);
-    s = yd * P.inv_dy + Comp<C>::shift_y;
+    s = fma(yd, P.inv_dy, Comp<C>::shift_y);
     f = floor(s);
     F.ty = s - f;
     F.ry = rel_base(f, h, j0);
     const int NZ = Comp<C>::centers ? P.nz + 2 : P.nz + 1;
-    const int m0 = locate_m0(P, Comp<C>::centers, face_cell(P, F.z), F.z);
+    const int m0 = locate_m0(Comp<C>::centers, half_cell(P, F.z));
     F.k0 = min(max(m0 - h, 0), NZ - O);
     return F;
 }
@@ -120,21 +120,23 @@ __device__ __forceinline__ double gather_box(const SlcParams &P, const double *b
     const double *dinv = Comp<C>::centers ? P.dinv_c[O] : P.dinv_f[O];
     z_weights<O, double>(zn, dinv, denom_rows(Comp<C>::centers, P.nz, O), F.k0, F.z, wz);
     const double *b = box + (ox * Box<O>::Y + oy) * Box<O>::Z + oz;
-    double acc = 0.0;
+    double acc[O];
+#pragma unroll
+    for (int k = 0; k < O; ++k) acc[k] = 0.0;
 #pragma unroll
     for (int i = 0; i < O; ++i) {
-        double accy = 0.0;
 #pragma unroll
         for (int j = 0; j < O; ++j) {
             const double *row = b + (i * Box<O>::Y + j) * Box<O>::Z;
-            double accz = 0.0;
+            const double w = wx[i] * wy[j];
 #pragma unroll
-            for (int k = 0; k < O; ++k) accz = fma(wz[k], row[k], accz);
-            accy = fma(wy[j], accz, accy);
+            for (int k = 0; k < O; ++k) acc[k] = fma(w, row[k], acc[k]);
         }
-        acc = fma(wx[i], accy, acc);
     }
-    return acc;
+    double r = 0.0;
+#pragma unroll
+    for (int k = 0; k < O; ++k) r = fma(wz[k], acc[k], r);
+    return r;
 }
 
 // Gather through L1 from the ghost-shaped array (the k_sl path).
@@ -143,7 +145,7 @@ __device__ __forceinline__ double gather_global(const SlcParams &P, NodeView<dou
                                                 double yd, const Foot &F)
 {
     Stencil<O, double> st;
-    build_stencil<C, O, double>(P, V.sx, V.sy, xd, yd, F.z, face_cell(P, F.z), st);
+    build_stencil<C, O, double>(P, V.sx, V.sy, xd, yd, F.z, half_cell(P, F.z), st);
     return gather_sum<O, double, double>(V.p, st);
 }
 
@@ -249,10 +251,7 @@ __global__ void __launch_bounds__(kThreads, Box<O>::min_blocks)
             ubb = gather_box<C, O>(P, boxM, Fm, Fm.rx - red[6], Fm.ry - red[8], Fm.k0 - Z0[1]);
         else
             ubb = gather_global<C, O>(P, ghost_view<double>(C, fnm1, P.nx, P.ny, P.nz), xm, ym, Fm);
-        const double Rn = xy_diffusion<C>(P, fn, i, j, k);
-        const double Rh = P.xy_lagged ? Rn : 2.0 * Rn - xy_diffusion<C>(P, fnm1, i, j, k);
-        double res = ubar * (4.0 / 3.0) + ubb * (-1.0 / 3.0);
-        res = res + ((2.0 / 3.0) * dt) * Rh;
+        const double res = bdf2_combine(ubar, ubb, dt, xy_diffusion_bdf2<C>(P, fn, fnm1, i, j, k));
         const GhostShape g = ghost_shape(C, P.nx, P.ny, P.nz);
         out[(size_t)(i + 1) * g.Y * g.Z + (size_t)(j + 1) * g.Z + (k + 1)] = res;
     }
@@ -391,10 +390,7 @@ __global__ void __launch_bounds__(kThreads, Box<O>::min_blocks)
             ubb = gather_box<C, O>(P, box, F, F.rx - red[6], F.ry - red[8], F.k0 - Z0);
         else
             ubb = gather_global<C, O>(P, ghost_view<double>(C, fnm1, P.nx, P.ny, P.nz), xd, yd, F);
-        const double Rn = xy_diffusion<C>(P, fn, i, j, k);
-        const double Rh = P.xy_lagged ? Rn : 2.0 * Rn - xy_diffusion<C>(P, fnm1, i, j, k);
-        double res = ubar * (4.0 / 3.0) + ubb * (-1.0 / 3.0);
-        res = res + ((2.0 / 3.0) * dt) * Rh;
+        const double res = bdf2_combine(ubar, ubb, dt, xy_diffusion_bdf2<C>(P, fn, fnm1, i, j, k));
         const GhostShape g = ghost_shape(C, P.nx, P.ny, P.nz);
         out[(size_t)(i + 1) * g.Y * g.Z + (size_t)(j + 1) * g.Z + (k + 1)] = res;
     }

@@ -65,10 +65,7 @@ __device__ __forceinline__ void sl_point(const SlcParams &P, const Vel3 &M,
         double xa, ya, za;
         arrival_point<C>(P, i, j, k, xa, ya, za);
         double Rh_early = 0.0;
-        if (MODE == 2 && RH_FIRST) {
-            const double Rn = xy_diffusion<C>(P, fn, i, j, k);
-            Rh_early = P.xy_lagged ? Rn : 2.0 * Rn - xy_diffusion<C>(P, fnm1, i, j, k);
-        }
+        if (MODE == 2 && RH_FIRST) Rh_early = xy_diffusion_bdf2<C>(P, fn, fnm1, i, j, k);
         double us0, vs0, ws0;
         first_sample<C, TO>(P, M, i, j, k, xa, ya, za, us0, vs0, ws0);
 
@@ -85,17 +82,11 @@ __device__ __forceinline__ void sl_point(const SlcParams &P, const Vel3 &M,
         if (MODE == 0) {
             res = ubar;
         } else if (MODE == 1) {
-            res = ubar + dt * xy_diffusion<C>(P, fn, i, j, k);
+            res = fma(dt, xy_diffusion<C>(P, fn, i, j, k), ubar);
         } else {
             const NodeView<double> Fm = ghost_view<double>(C, fnm1, P.nx, P.ny, P.nz);
             const double ubb = gather_foot<C, O>(P, Fm, xf, yf, zf, ncl);
-            double Rh = Rh_early;
-            if (!RH_FIRST) {
-                const double Rn = xy_diffusion<C>(P, fn, i, j, k);
-                Rh = P.xy_lagged ? Rn : 2.0 * Rn - xy_diffusion<C>(P, fnm1, i, j, k);
-            }
-            res = ubar * (4.0 / 3.0) + ubb * (-1.0 / 3.0);
-            res = res + ((2.0 / 3.0) * dt) * Rh;
+            res = bdf2_combine(ubar, ubb, dt, RH_FIRST ? Rh_early : xy_diffusion_bdf2<C>(P, fn, fnm1, i, j, k));
         }
         const GhostShape g = ghost_shape(C, P.nx, P.ny, P.nz);
         out[(size_t)(i + 1) * g.Y * g.Z + (size_t)(j + 1) * g.Z + (k + 1)] = res;
@@ -199,7 +190,7 @@ __global__ void __launch_bounds__(kThreads) k_advect_multi(const __grid_constant
         trace_foot<TO>(P, M, xa, ya, za, 0.5 * dt, us0, vs0, ws0, xd, yd, zd);
         if (zd < P.z_lo || zd > P.z_hi) ncl += 1;
         const double z = clampz(P, zd);
-        const int c = face_cell(P, z);
+        const int c = half_cell(P, z);
         const NodeView<double> V0 = ghost_view<double>(C, F.in[0], P.nx, P.ny, P.nz);
         Stencil<O, double> st;
         build_stencil<C, O, double>(P, V0.sx, V0.sy, xd, yd, z, c, st);
@@ -250,7 +241,7 @@ __global__ void __launch_bounds__(kThreads) k_interp(SlcParams P, NodeView<doubl
             if (zz < P.z_lo || zz > P.z_hi) ncl = 1;
             zz = clampz(P, zz);
         }
-        int c = face_cell(P, zz);
+        const int c = half_cell(P, zz);
         Stencil<O, double> st;
         build_stencil<C, O, double>(P, F.sx, F.sy, x[p], y[p], zz, c, st);
         out[p] = gather_sum<O, double, double>(F.p, st);

@@ -78,6 +78,45 @@ int upload(slc_grid *g, T **p, const std::vector<T> &h, const char *what)
     return SLC_OK;
 }
 
+// Tables of half_cell: the edges of the half cells (the tanh map's faces,
+// utils.py:21-61, and the centres between them), and per bin of height
+// Lz / nbins the half cell that holds the bin's lower edge.  The bins are a
+// tenth lower than the lowest half cell and their edges are taken a hair low,
+// so that rounding in z * scale cannot skip an edge.  Empty where the centres
+// do not lie between the map's faces, or where more than 65536 bins would be
+// needed.
+void half_cell_bins(const SlcParams &P, const std::vector<double> &zc, std::vector<double> &edges,
+                    std::vector<unsigned short> &bins)
+{
+    edges.resize((size_t)2 * P.nz + 1);
+    for (int k = 0; k <= P.nz; ++k) {
+        const double s = (double)k / P.nz;
+        edges[2 * k] = P.symmetric ? 0.5 * P.Lz * (1.0 + std::tanh(P.gamma * (2.0 * s - 1.0)) / P.tanh_g)
+                                   : P.Lz * (1.0 - std::tanh(P.gamma * (1.0 - s)) / P.tanh_g);
+        if (k < P.nz) edges[2 * k + 1] = zc[k + 1];
+    }
+    double dz = P.Lz;
+    for (int m = 0; m < 2 * P.nz; ++m) dz = std::min(dz, edges[m + 1] - edges[m]);
+    bins.clear();
+    if (!(dz > P.Lz / 58000.0)) return;
+    const int n = (int)std::ceil(P.Lz / (0.9 * dz));
+    bins.resize((size_t)n);
+    int m = 0;
+    for (int b = 0; b < n; ++b) {
+        const double edge = P.Lz * ((double)b / n) - 1e-12 * P.Lz;
+        while (m < 2 * P.nz - 1 && edges[m + 1] <= edge) ++m;
+        bins[b] = (unsigned short)m;
+    }
+}
+
+// {node, 1 / interval above it} of every node but the last.
+std::vector<double2> linear_table(const std::vector<double> &zn)
+{
+    std::vector<double2> t(zn.size() - 1);
+    for (size_t k = 0; k < t.size(); ++k) t[k] = make_double2(zn[k], 1.0 / (zn[k + 1] - zn[k]));
+    return t;
+}
+
 // semilag.py:102-114: 1 / prod_{l != m}(z[b+m] - z[b+l]), products in ascending l,
 // stored node-major (entry (b, m) at m * nb + b).
 std::vector<double> denom_table(const std::vector<double> &zn, int order)
@@ -538,6 +577,8 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     P.dy = d->Ly / ny;
     P.inv_dx = 1.0 / P.dx;
     P.inv_dy = 1.0 / P.dy;
+    P.inv_nx = 1.0 / nx;
+    P.inv_ny = 1.0 / ny;
     P.inv_dx2 = 1.0 / (P.dx * P.dx);
     P.inv_dy2 = 1.0 / (P.dy * P.dy);
     P.Lz = d->Lz;
@@ -585,6 +626,26 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
         std::vector<float> zc32(zc.begin(), zc.end()), zf32(zf.begin(), zf.end());
         CREATE_CK(upload(g, &g->zc32, zc32, "z_c fp32"));
         CREATE_CK(upload(g, &g->zf32, zf32, "z_f fp32"));
+    }
+    {
+        std::vector<double> edges;
+        std::vector<unsigned short> bins;
+        half_cell_bins(P, zc, edges, bins);
+        if (!bins.empty()) {
+            double *half = nullptr;
+            unsigned short *bin = nullptr;
+            CREATE_CK(upload(g, &half, edges, "half-cell edges"));
+            CREATE_CK(upload(g, &bin, bins, "half-cell bins"));
+            P.zhalf = half;
+            P.zbin = bin;
+            P.zbins = (int)bins.size();
+            P.zbin_scale = P.zbins / P.Lz;
+        }
+        double2 *lin = nullptr;
+        CREATE_CK(upload(g, &lin, linear_table(zc), "centre intervals"));
+        P.lin_c = lin;
+        CREATE_CK(upload(g, &lin, linear_table(zf), "face intervals"));
+        P.lin_f = lin;
     }
     for (int o = 2; o <= SLC_MAX_ORDER; o += 2) {
         if (nz + 2 - o + 1 <= 0) continue;

@@ -18,6 +18,7 @@ struct SlcParams {
     int top_neumann;   // free-slip top wall for u, v
     int xy_lagged;     // BDF2 explicit xy-rhs: 0 extrap (2R^n - R^{n-1}), 1 lagged (R^n)
     double dx, dy, inv_dx, inv_dy, inv_dx2, inv_dy2;
+    double inv_nx, inv_ny;  // 1 / nx, 1 / ny (wrap_base)
     double Lz, two_over_Lz, inv_Lz;
     double gamma, inv_gamma, tanh_g, half_nz, nzd;
     double z_lo, z_hi;  // departure z kept in [z_lo, z_hi] (semilag.py:244-247)
@@ -31,6 +32,16 @@ struct SlcParams {
     const float *dinv_c32[SLC_MAX_ORDER + 1];  // FP32 copies for the mixed form
     const float *dinv_f32[SLC_MAX_ORDER + 1];
     const float *zc32, *zf32;
+    // cell lookup (half_cell): zbins bins of equal height over [0, Lz], each with
+    // the half cell its lower edge lies in, and the half cells' lower edges
+    // (the tanh map's faces, z_c between them); null where the bins would be
+    // too many (the map is inverted then)
+    const unsigned short *zbin;
+    const double *zhalf;
+    double zbin_scale;  // zbins / Lz
+    int zbins;
+    // linear interpolation in z: {node, 1 / interval above it} per node
+    const double2 *lin_c, *lin_f;
     double udenom[SLC_MAX_ORDER + 1][SLC_MAX_ORDER];  // semilag.py:117-127
 };
 
@@ -112,17 +123,27 @@ __device__ __forceinline__ int wrap_index(int i, int n)
     return i;
 }
 
-__device__ __forceinline__ int wrap_base(double f, int n)
+// f = floor(s), an integer-valued double, reduced to [0, n); NaN and huge
+// values end in [0, n) too, so indices never leave the array.  Branch-free, so
+// that the loads of a point's samples can be issued across it: inv_n = 1 / n
+// rounded may put the quotient one off, which the integer corrections undo.
+__device__ __forceinline__ int wrap_base(double f, int n, double inv_n)
 {
-    // f = floor(s), an integer-valued double.  Fast path: already in [0, n)
-    // (every foot within a period); otherwise reduce with floor division.
-    // NaN or huge values end in [0, n) too, so indices never leave the array.
-    const double dn = (double)n;
-    if (f >= 0.0 && f < dn) return (int)f;
-    double r = f - dn * floor(f / dn);
-    if (!(r >= 0.0)) r = 0.0;
-    if (r >= dn) r = dn - 1.0;
-    return (int)r;
+    int i = (int)fma(-(double)n, floor(f * inv_n), f);
+    i += (i < 0) ? n : 0;
+    i -= (i >= n) ? n : 0;
+    return min(max(i, 0), n - 1);
+}
+
+// The trajectory, stencil-location and epilogue arithmetic below is written
+// with explicit fma / __dmul_rn, so every kernel that inlines it rounds alike:
+// left to contraction, ptxas may fuse the same expression differently in two
+// kernels, and the staged and the L1 gathers would differ in the last bit.
+
+// a b + c d with the first product rounded.
+__device__ __forceinline__ double dot2(double a, double b, double c, double d)
+{
+    return fma(c, d, __dmul_rn(a, b));
 }
 
 // Continuous face index kf in [0, nz] of a physical z: analytic inverse of
@@ -131,30 +152,41 @@ __device__ __forceinline__ double face_coord(const SlcParams &P, double z)
 {
     const double lo = -1.0 + 1e-15, hi = 1.0 - 1e-15;
     if (P.symmetric) {
-        double arg = (z * P.two_over_Lz - 1.0) * P.tanh_g;
+        double arg = __dmul_rn(fma(z, P.two_over_Lz, -1.0), P.tanh_g);
         arg = fmin(fmax(arg, lo), hi);
-        return (atanh(arg) * P.inv_gamma + 1.0) * P.half_nz;
+        return __dmul_rn(fma(atanh(arg), P.inv_gamma, 1.0), P.half_nz);
     } else {
-        double arg = (1.0 - z * P.inv_Lz) * P.tanh_g;
+        double arg = __dmul_rn(fma(-z, P.inv_Lz, 1.0), P.tanh_g);
         arg = fmin(fmax(arg, lo), hi);
-        return (1.0 - atanh(arg) * P.inv_gamma) * P.nzd;
+        return __dmul_rn(fma(-atanh(arg), P.inv_gamma, 1.0), P.nzd);
     }
 }
 
-// Face cell c = clamp(floor(kf), 0, nz-1) (semilag.py:413-416).
-__device__ __forceinline__ int face_cell(const SlcParams &P, double z)
+// Half cell of z: 2 c + 1 where z is at or above the centre of its face cell
+// c, 2 c below it, with c = clamp(floor(kf), 0, nz-1) (semilag.py:413-416), kf
+// the continuous face index.  Four cells are located per arrival point (a
+// trajectory sample and a foot at both depths), and inverting the map with
+// atanh is a chain of some hundred dependent FP64 operations each time.  The
+// bins are lower than the lowest half cell, so a bin holds at most one edge:
+// one lookup and one comparison give the same cell (a z within rounding of a
+// face may land on either side of it, where the interpolants of both cells
+// agree).
+__device__ __forceinline__ int half_cell(const SlcParams &P, double z)
 {
+    if (P.zbin) {
+        const int b = min(max((int)(z * P.zbin_scale), 0), P.zbins - 1);  // NaN -> 0
+        const int m = __ldg(P.zbin + b);
+        return min(m + (z >= __ldg(P.zhalf + m + 1) ? 1 : 0), 2 * P.nz - 1);
+    }
     double kf = floor(face_coord(P, z));
     kf = fmin(fmax(kf, 0.0), (double)(P.nz - 1));  // NaN -> 0
-    return (int)kf;
+    const int c = (int)kf;
+    return 2 * c + (z >= __ldg(P.zc + c + 1) ? 1 : 0);
 }
 
-// Interval index m0 with znodes[m0] <= z < znodes[m0+1] (semilag.py:417-420).
-__device__ __forceinline__ int locate_m0(const SlcParams &P, bool centers, int c, double z)
-{
-    if (!centers) return c;
-    return c + (z >= __ldg(P.zc + c + 1) ? 1 : 0);
-}
+// Interval index m0 with znodes[m0] <= z < znodes[m0+1] (semilag.py:417-420),
+// of the centres (u, v) or the faces (w), from the half cell.
+__device__ __forceinline__ int locate_m0(bool centers, int half) { return centers ? (half + 1) >> 1 : half >> 1; }
 
 // Lagrange weights on the integer offsets m - (O/2 - 1), t in [0, 1)
 // (semilag.py:426-439), via prefix/suffix products.
@@ -219,27 +251,27 @@ struct Stencil {
 
 template <int C, int O, typename T>
 __device__ __forceinline__ void build_stencil(const SlcParams &P, int sx, int sy, double x, double y,
-                                              double z, int c_face, Stencil<O, T> &st)
+                                              double z, int half, Stencil<O, T> &st)
 {
     constexpr int h = O / 2 - 1;
     const int NZ = Comp<C>::centers ? P.nz + 2 : P.nz + 1;
-    double s = x * P.inv_dx + Comp<C>::shift_x;
+    double s = fma(x, P.inv_dx, Comp<C>::shift_x);
     double f = floor(s);
     T t = (T)(s - f);
-    int b = wrap_base(f, P.nx);
+    int b = wrap_base(f, P.nx, P.inv_nx);
 #pragma unroll
     for (int m = 0; m < O; ++m) st.xoff[m] = wrap_index(b + m - h, P.nx) * sx;
     uniform_weights<O, T>(P, t, st.wx);
 
-    s = y * P.inv_dy + Comp<C>::shift_y;
+    s = fma(y, P.inv_dy, Comp<C>::shift_y);
     f = floor(s);
     t = (T)(s - f);
-    b = wrap_base(f, P.ny);
+    b = wrap_base(f, P.ny, P.inv_ny);
 #pragma unroll
     for (int m = 0; m < O; ++m) st.yoff[m] = wrap_index(b + m - h, P.ny) * sy;
     uniform_weights<O, T>(P, t, st.wy);
 
-    int m0 = locate_m0(P, Comp<C>::centers, c_face, z);
+    int m0 = locate_m0(Comp<C>::centers, half);
     int k0 = min(max(m0 - h, 0), NZ - O);
     st.k0 = k0;
     const double *zn = Comp<C>::centers ? P.zc : P.zf;
@@ -253,27 +285,31 @@ __device__ __forceinline__ void build_stencil(const SlcParams &P, int sx, int sy
     }
 }
 
-// Separable tensor-product contraction: z first (O^3 FMAs), then y, then x
-// (the reference sums the O^3 products in one sequence, semilag.py:44-59;
-// the grouping here differs only by rounding).
+// Separable tensor-product contraction: the rows' x and y weights are multiplied
+// and every z node's sum runs over the rows (O independent chains of fused
+// multiply-adds), the z weights come last (the reference sums the O^3 products
+// in one sequence, semilag.py:44-59; the grouping here differs only by
+// rounding).
 template <int O, typename T, typename A>
 __device__ __forceinline__ A gather_sum(const T *__restrict__ F, const Stencil<O, T> &st)
 {
-    A acc = (A)0;
+    A acc[O];
+#pragma unroll
+    for (int k = 0; k < O; ++k) acc[k] = (A)0;
 #pragma unroll
     for (int i = 0; i < O; ++i) {
-        A accy = (A)0;
 #pragma unroll
         for (int j = 0; j < O; ++j) {
             const T *row = F + st.xoff[i] + st.yoff[j] + st.k0;
-            A accz = (A)0;
+            const A w = (A)st.wx[i] * (A)st.wy[j];
 #pragma unroll
-            for (int k = 0; k < O; ++k) accz = fma((A)st.wz[k], (A)__ldg(row + k), accz);
-            accy = fma((A)st.wy[j], accz, accy);
+            for (int k = 0; k < O; ++k) acc[k] = fma(w, (A)__ldg(row + k), acc[k]);
         }
-        acc = fma((A)st.wx[i], accy, acc);
     }
-    return acc;
+    A r = (A)0;
+#pragma unroll
+    for (int k = 0; k < O; ++k) r = fma((A)st.wz[k], acc[k], r);
+    return r;
 }
 
 // One trilinear sample of node view V from precomputed corner indices and
@@ -286,12 +322,12 @@ __device__ __forceinline__ double tri_sample(NodeView<T> V, int i0, int i1, doub
     const T *p01 = V.p + i0 * V.sx + j1 * V.sy + k0;
     const T *p10 = V.p + i1 * V.sx + j0 * V.sy + k0;
     const T *p11 = V.p + i1 * V.sx + j1 * V.sy + k0;
-    const double a00 = wz0 * (double)__ldg(p00) + wz1 * (double)__ldg(p00 + 1);
-    const double a01 = wz0 * (double)__ldg(p01) + wz1 * (double)__ldg(p01 + 1);
-    const double a10 = wz0 * (double)__ldg(p10) + wz1 * (double)__ldg(p10 + 1);
-    const double a11 = wz0 * (double)__ldg(p11) + wz1 * (double)__ldg(p11 + 1);
+    const double a00 = dot2(wz0, (double)__ldg(p00), wz1, (double)__ldg(p00 + 1));
+    const double a01 = dot2(wz0, (double)__ldg(p01), wz1, (double)__ldg(p01 + 1));
+    const double a10 = dot2(wz0, (double)__ldg(p10), wz1, (double)__ldg(p10 + 1));
+    const double a11 = dot2(wz0, (double)__ldg(p11), wz1, (double)__ldg(p11 + 1));
     const double wx0 = 1.0 - tx, wy0 = 1.0 - ty;
-    return wx0 * (wy0 * a00 + ty * a01) + tx * (wy0 * a10 + ty * a11);
+    return dot2(wx0, dot2(wy0, a00, ty, a01), tx, dot2(wy0, a10, ty, a11));
 }
 
 // The pieces of the three trilinear stencils at one point that the staggered
@@ -307,40 +343,36 @@ struct TriShared {
 };
 
 __device__ __forceinline__ void tri_shared(const SlcParams &P, double x, double y, double z,
-                                           int c_face, TriShared &t)
+                                           int half, TriShared &t)
 {
-    double sa = x * P.inv_dx;
+    double sa = __dmul_rn(x, P.inv_dx);
     double f = floor(sa);
     t.txa = sa - f;
-    t.ia0 = wrap_base(f, P.nx);
+    t.ia0 = wrap_base(f, P.nx, P.inv_nx);
     t.ia1 = (t.ia0 + 1 == P.nx) ? 0 : t.ia0 + 1;
     double sb = sa - 0.5;
     f = floor(sb);
     t.txb = sb - f;
-    t.ib0 = wrap_base(f, P.nx);
+    t.ib0 = wrap_base(f, P.nx, P.inv_nx);
     t.ib1 = (t.ib0 + 1 == P.nx) ? 0 : t.ib0 + 1;
-    sa = y * P.inv_dy;
+    sa = __dmul_rn(y, P.inv_dy);
     f = floor(sa);
     t.tya = sa - f;
-    t.ja0 = wrap_base(f, P.ny);
+    t.ja0 = wrap_base(f, P.ny, P.inv_ny);
     t.ja1 = (t.ja0 + 1 == P.ny) ? 0 : t.ja0 + 1;
     sb = sa - 0.5;
     f = floor(sb);
     t.tyb = sb - f;
-    t.jb0 = wrap_base(f, P.ny);
+    t.jb0 = wrap_base(f, P.ny, P.inv_ny);
     t.jb1 = (t.jb0 + 1 == P.ny) ? 0 : t.jb0 + 1;
-    // centres: interval m0 = c + (z >= zc[c+1]), clamped to [0, nz]; faces: c in [0, nz-1]
-    int kc = c_face + (z >= __ldg(P.zc + c_face + 1) ? 1 : 0);
-    kc = min(max(kc, 0), P.nz);
-    const int kf = min(max(c_face, 0), P.nz - 1);
-    t.kc = kc;
-    t.kf = kf;
-    const double *dc = P.dinv_c[2] + kc;  // order-2 tables: nz+1 / nz rows
-    const double *df = P.dinv_f[2] + kf;
-    t.wc0 = (z - __ldg(P.zc + kc + 1)) * __ldg(dc);
-    t.wc1 = (z - __ldg(P.zc + kc)) * __ldg(dc + P.nz + 1);
-    t.wf0 = (z - __ldg(P.zf + kf + 1)) * __ldg(df);
-    t.wf1 = (z - __ldg(P.zf + kf)) * __ldg(df + P.nz);
+    // centres: interval (half + 1) / 2 in [0, nz]; faces: half / 2 in [0, nz-1]
+    t.kc = locate_m0(true, half);
+    t.kf = locate_m0(false, half);
+    const double2 lc = __ldg(P.lin_c + t.kc), lf = __ldg(P.lin_f + t.kf);
+    t.wc1 = __dmul_rn(z - lc.x, lc.y);
+    t.wc0 = 1.0 - t.wc1;
+    t.wf1 = __dmul_rn(z - lf.x, lf.y);
+    t.wf0 = 1.0 - t.wf1;
 }
 
 // Node value accessor for the arrival-point sample below (FP64 node views).
@@ -369,31 +401,25 @@ __device__ __forceinline__ void arrival_sample(const SlcParams &P, const V3 &M, 
         us = val(M.u, ip, j, k + 1);
         vs = 0.25 * ((val(M.v, i, j, k + 1) + val(M.v, ip, j, k + 1)) +
                      (val(M.v, i, jp, k + 1) + val(M.v, ip, jp, k + 1)));
-        const double z = __ldg(P.zc + k + 1);
-        const double *df = P.dinv_f[2] + k;  // face interval k
-        const double w0 = (z - __ldg(P.zf + k + 1)) * __ldg(df);
-        const double w1 = (z - __ldg(P.zf + k)) * __ldg(df + P.nz);
-        ws = 0.5 * ((w0 * val(M.w, i, j, k) + w1 * val(M.w, i, j, k + 1)) +
-                    (w0 * val(M.w, ip, j, k) + w1 * val(M.w, ip, j, k + 1)));
+        const double2 lf = __ldg(P.lin_f + k);  // face interval k
+        const double w1 = __dmul_rn(__ldg(P.zc + k + 1) - lf.x, lf.y), w0 = 1.0 - w1;
+        ws = 0.5 * (dot2(w0, val(M.w, i, j, k), w1, val(M.w, i, j, k + 1)) +
+                    dot2(w0, val(M.w, ip, j, k), w1, val(M.w, ip, j, k + 1)));
     } else if (C == 1) {
         us = 0.25 * ((val(M.u, i, j, k + 1) + val(M.u, ip, j, k + 1)) +
                      (val(M.u, i, jp, k + 1) + val(M.u, ip, jp, k + 1)));
         vs = val(M.v, i, jp, k + 1);
-        const double z = __ldg(P.zc + k + 1);
-        const double *df = P.dinv_f[2] + k;
-        const double w0 = (z - __ldg(P.zf + k + 1)) * __ldg(df);
-        const double w1 = (z - __ldg(P.zf + k)) * __ldg(df + P.nz);
-        ws = 0.5 * ((w0 * val(M.w, i, j, k) + w1 * val(M.w, i, j, k + 1)) +
-                    (w0 * val(M.w, i, jp, k) + w1 * val(M.w, i, jp, k + 1)));
+        const double2 lf = __ldg(P.lin_f + k);
+        const double w1 = __dmul_rn(__ldg(P.zc + k + 1) - lf.x, lf.y), w0 = 1.0 - w1;
+        ws = 0.5 * (dot2(w0, val(M.w, i, j, k), w1, val(M.w, i, j, k + 1)) +
+                    dot2(w0, val(M.w, i, jp, k), w1, val(M.w, i, jp, k + 1)));
     } else {
-        const double z = __ldg(P.zf + k + 1);
-        const double *dc = P.dinv_c[2] + (k + 1);  // centre interval k+1
-        const double c0 = (z - __ldg(P.zc + k + 2)) * __ldg(dc);
-        const double c1 = (z - __ldg(P.zc + k + 1)) * __ldg(dc + P.nz + 1);
-        us = 0.5 * ((c0 * val(M.u, i, j, k + 1) + c1 * val(M.u, i, j, k + 2)) +
-                    (c0 * val(M.u, ip, j, k + 1) + c1 * val(M.u, ip, j, k + 2)));
-        vs = 0.5 * ((c0 * val(M.v, i, j, k + 1) + c1 * val(M.v, i, j, k + 2)) +
-                    (c0 * val(M.v, i, jp, k + 1) + c1 * val(M.v, i, jp, k + 2)));
+        const double2 lc = __ldg(P.lin_c + k + 1);  // centre interval k+1
+        const double c1 = __dmul_rn(__ldg(P.zf + k + 1) - lc.x, lc.y), c0 = 1.0 - c1;
+        us = 0.5 * (dot2(c0, val(M.u, i, j, k + 1), c1, val(M.u, i, j, k + 2)) +
+                    dot2(c0, val(M.u, ip, j, k + 1), c1, val(M.u, ip, j, k + 2)));
+        vs = 0.5 * (dot2(c0, val(M.v, i, j, k + 1), c1, val(M.v, i, j, k + 2)) +
+                    dot2(c0, val(M.v, i, jp, k + 1), c1, val(M.v, i, jp, k + 2)));
         ws = val(M.w, i, j, k + 1);
     }
 }
@@ -406,16 +432,16 @@ __device__ __forceinline__ void arrival_point(const SlcParams &P, int i, int j, 
 {
     double ar = (double)(i + 1), aj = (double)(j + 1);
     if (C == 0) {
-        xa = ar * P.dx;
-        ya = (aj - 0.5) * P.dy;
+        xa = __dmul_rn(ar, P.dx);
+        ya = __dmul_rn(aj - 0.5, P.dy);
         za = __ldg(P.zc + k + 1);
     } else if (C == 1) {
-        xa = (ar - 0.5) * P.dx;
-        ya = aj * P.dy;
+        xa = __dmul_rn(ar - 0.5, P.dx);
+        ya = __dmul_rn(aj, P.dy);
         za = __ldg(P.zc + k + 1);
     } else {
-        xa = (ar - 0.5) * P.dx;
-        ya = (aj - 0.5) * P.dy;
+        xa = __dmul_rn(ar - 0.5, P.dx);
+        ya = __dmul_rn(aj - 0.5, P.dy);
         za = __ldg(P.zf + k + 1);
     }
 }
