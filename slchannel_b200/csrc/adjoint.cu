@@ -14,7 +14,8 @@
 //    the same rfft2 / per-(kx, ky) tridiagonal / irfft2 pipeline with every
 //    column's system transposed (the Fourier basis diagonalises the x, y
 //    part and the coefficients are real);
-//  * z-solve A^-1: A^-T per column (sequential Thomas on the transpose);
+//  * z-solve A^-1: A^-T per column (the forward's solve with the transposed
+//    systems' factors);
 //  * SL: the gather's transpose is a deterministic segmented scatter-add.
 //    Each foot becomes a record (stencil base, fractional position,
 //    coefficient); records are counting-sorted by base (ties by record id),
@@ -835,72 +836,6 @@ __global__ void k_gradT_pack(SlcParams P, const double *__restrict__ lu, const d
     psi[t] = s;
 }
 
-// Transposed Thomas sweep per (kx, ky) column (the forward's rows, with the
-// sub- and super-diagonals exchanged), 1/(nx ny) folded in.
-__global__ void __launch_bounds__(kT) k_thomas_T(SlcParams P, double *__restrict__ hat,
-                                                 double *__restrict__ cpw, const double *__restrict__ kx2,
-                                                 const double *__restrict__ ky2,
-                                                 const double *__restrict__ cl,
-                                                 const double *__restrict__ cr, double norm)
-{
-    const int nky = P.ny / 2 + 1;
-    const int ncol = P.nx * nky;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int col = t >> 1, part = t & 1;
-    const bool active = col < ncol;
-    const int nz = P.nz;
-    const size_t st = 2 * (size_t)ncol;
-    double *h = hat + 2 * (size_t)(active ? col : 0) + part;
-    double *cpc = cpw + (active ? col : 0);
-    double k2 = 0.0;
-    if (active) {
-        const int kx = col / nky, ky = col - (col / nky) * nky;
-        k2 = kx2[kx] + ky2[ky];
-    }
-    auto rows = [&](int k, double &a, double &b, double &c) {
-        a = k > 0 ? cl[k] : 0.0;
-        b = -(cl[k] + cr[k] + k2);
-        if (k == 0) b += cl[0];
-        if (k == nz - 1) b += cr[nz - 1];
-        c = k < nz - 1 ? cr[k] : 0.0;
-        if (col == 0 && k == 0) {
-            b = 1.0;
-            c = 0.0;
-        }
-    };
-    if (active) {
-        double cprev = 0.0, dprev = 0.0;
-        for (int k = 0; k < nz; ++k) {
-            double a, b, c, an, bn, cn, ap, bp, cpv;
-            rows(k, a, b, c);
-            // transpose: sub_k = c_{k-1}, super_k = a_{k+1}
-            double sub = 0.0, sup = 0.0;
-            if (k > 0) {
-                rows(k - 1, ap, bp, cpv);
-                sub = cpv;
-            }
-            if (k < nz - 1) {
-                rows(k + 1, an, bn, cn);
-                sup = an;
-            }
-            const double id = 1.0 / (b - sub * cprev);
-            cprev = sup * id;
-            dprev = (h[k * st] - sub * dprev) * id;
-            h[k * st] = dprev;
-            if (part == 0) cpc[k * (size_t)ncol] = cprev;
-        }
-    }
-    __syncwarp();
-    if (active) {
-        double x = 0.0;
-        for (int k = nz - 1; k >= 0; --k) {
-            const double dk = h[k * st];
-            x = (k == nz - 1) ? dk : dk - cpc[k * (size_t)ncol] * x;
-            h[k * st] = x * norm;
-        }
-    }
-}
-
 // lam -= c * D^T phi (phi z-major), D the forward's divergence (utils.py:166-180).
 __global__ void k_divT(SlcParams P, const double *__restrict__ phi, const double *__restrict__ dz_f,
                        double c, double *lu, double *lv, double *lw)
@@ -925,74 +860,6 @@ __global__ void k_divT(SlcParams P, const double *__restrict__ phi, const double
             c * (f0 / dz_f[k] - F(i, j, k + 1) / dz_f[k + 1]);
 }
 
-// ---- z-solve transpose: A^T x = d per column -----------------------------------
-__global__ void k_zsolve_T(SlcParams P, const double *__restrict__ dz_c, const double *__restrict__ dz_f,
-                           double dt, double *lu, double *lv, double *lw, double *scratch)
-{
-    const long long ncol = (long long)P.nx * P.ny;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * ncol) return;
-    const int comp = (int)(t / ncol);
-    const int col = (int)(t % ncol);
-    const int i = col / P.ny, j = col % P.ny;
-    const GhostShape g = ghost_shape(comp, P.nx, P.ny, P.nz);
-    double *base = comp == 0 ? lu : (comp == 1 ? lv : lw);
-    double *x = base + (size_t)(i + 1) * g.Y * g.Z + (size_t)(j + 1) * g.Z + 1;
-    const int which = comp == 2 ? 1 : 0;
-    const int n = which == 0 ? P.nz : P.nz - 1;
-    const double alpha = 1.0 * dt * P.nu;
-    auto rows = [&](int k, double &a, double &b, double &c) {
-        double dl, dr, dc;
-        if (which == 0) {
-            dl = dz_c[k];
-            dr = dz_c[k + 1];
-            dc = dz_f[k];
-        } else {
-            dl = dz_f[k];
-            dr = dz_f[k + 1];
-            dc = dz_c[k + 1];
-        }
-        const double lower = -alpha / (dl * dc);
-        const double center = 1.0 + alpha * (1.0 / dl + 1.0 / dr) / dc;
-        const double upper = -alpha / (dr * dc);
-        a = lower;
-        b = center;
-        c = upper;
-        if (k == 0) {
-            a = 0.0;
-            if (which == 0) b = center - lower;
-        }
-        if (k == n - 1) {
-            c = 0.0;
-            if (which == 0) b = P.top_neumann ? center + upper : center - upper;
-        }
-    };
-    double cprev = 0.0, dprev = 0.0;
-    for (int k = 0; k < n; ++k) {
-        double a, b, c, a2, b2, c2;
-        rows(k, a, b, c);
-        double sub = 0.0, sup = 0.0;
-        if (k > 0) {
-            rows(k - 1, a2, b2, c2);
-            sub = c2;
-        }
-        if (k < n - 1) {
-            rows(k + 1, a2, b2, c2);
-            sup = a2;
-        }
-        const double id = 1.0 / (b - sub * cprev);
-        cprev = sup * id;
-        dprev = (x[k] - sub * dprev) * id;
-        x[k] = dprev;
-        scratch[(size_t)k * 3 * ncol + t] = cprev;
-    }
-    double y = 0.0;
-    for (int k = n - 1; k >= 0; --k) {
-        y = (k == n - 1) ? x[k] : x[k] - scratch[(size_t)k * 3 * ncol + t] * y;
-        x[k] = y;
-    }
-}
-
 __global__ void k_axpy(double *y, const double *__restrict__ x, double a, long long n)
 {
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
@@ -1011,7 +878,9 @@ struct AdjWS {
     int *keys = nullptr, *order = nullptr, *counts = nullptr, *starts = nullptr, *fill = nullptr;
     int *sums = nullptr, *total = nullptr;
     double *lam_mid[3] = {nullptr, nullptr, nullptr};
-    double *scratch = nullptr, *partials = nullptr, *S = nullptr;
+    double *zs_tab = nullptr, zs_dt = 0.0;  // z-solve tables of the transposed systems, at zs_dt
+    double *th_id = nullptr, *th_g = nullptr;  // Poisson factors of the transposed systems
+    double *partials = nullptr, *S = nullptr;
     double *W = nullptr;  // sorted gather weights, 3 O arrays of n_c[0]
     int *kz = nullptr;    // sorted gather records' first z node
     double *Stri = nullptr;  // trilinear corner partials, 8 arrays of nkeys_max
@@ -1042,7 +911,7 @@ int adj_alloc(slc_grid *g, T **p, size_t n, const char *what)
     return SLC_OK;
 }
 
-int ensure_adj(slc_grid *g)
+int ensure_adj(slc_grid *g, cudaStream_t s)
 {
     if (g->adj) return SLC_OK;
     const SlcParams &P = g->P;
@@ -1067,15 +936,24 @@ int ensure_adj(slc_grid *g)
     if (!rc) rc = adj_alloc(g, &w->sums, (size_t)nb, "adjoint scan sums");
     if (!rc) rc = adj_alloc(g, &w->total, (size_t)1, "adjoint scan total");
     for (int c = 0; c < 3 && !rc; ++c) rc = adj_alloc(g, &w->lam_mid[c], g->ghost_elems[c], "adjoint U*");
-    if (!rc) rc = adj_alloc(g, &w->scratch, (size_t)3 * plane * P.nz, "adjoint z-solve scratch");
+    if (!rc) rc = adj_alloc(g, &w->zs_tab, zsolve_table_doubles(P.nz), "adjoint z-solve tables");
     if (!rc) rc = adj_alloc(g, &w->partials, (size_t)kSumBlocks, "adjoint partials");
     if (!rc) rc = adj_alloc(g, &w->S, (size_t)1, "adjoint sum");
     if (!rc) rc = adj_alloc(g, &w->W, (size_t)3 * SLC_MAX_ORDER * w->n_c[0], "adjoint gather weights");
     if (!rc) rc = adj_alloc(g, &w->kz, (size_t)w->n_c[0], "adjoint gather z bases");
     if (!rc) rc = adj_alloc(g, &w->Stri, (size_t)8 * w->nkeys_max, "adjoint trilinear partials");
+    const size_t ncplx = (size_t)P.nz * P.nx * (P.ny / 2 + 1);
+    if (!rc) rc = adj_alloc(g, &w->th_id, ncplx, "adjoint Poisson factors");
+    if (!rc) rc = adj_alloc(g, &w->th_g, ncplx, "adjoint Poisson factors");
     if (rc) {
         delete w;
         return rc;
+    }
+    cudaError_t e = launch_thomas_factors(P, w->th_id, w->th_g, g->kx2, g->ky2, g->cl, g->cr, true, s);
+    if (e != cudaSuccess) {
+        delete w;
+        g->err = std::string("adjoint Poisson factors: ") + cudaGetErrorString(e);
+        return SLC_E_CUDA;
     }
     g->adj = w;
     return SLC_OK;
@@ -1250,7 +1128,7 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
     }
     cudaSetDevice(g->device);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = ensure_adj(g);
+    int rc = ensure_adj(g, s);
     if (rc) return rc;
     AdjWS *w = g->adj;
     const SlcParams &P = g->P;
@@ -1274,12 +1152,7 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
         g->err = "cufftExecD2Z (adjoint)";
         return SLC_E_CUFFT;
     }
-    {
-        const long long nthr = 2LL * P.nx * (P.ny / 2 + 1);
-        const double norm = 1.0 / ((double)P.nx * (double)P.ny);
-        k_thomas_T<<<nblk(nthr), kT, 0, s>>>(P, g->hat, g->cpw, g->kx2, g->ky2, g->cl, g->cr, norm);
-        count_launches(1);
-    }
+    ADJ_CK(launch_thomas_poisson(P, g->hat, w->th_id, w->th_g, g->cl, g->cr, s, true), "Poisson Thomas adjoint");
     if (cufftSetStream(g->inv, s) != CUFFT_SUCCESS ||
         cufftExecZ2D(g->inv, (cufftDoubleComplex *)g->hat, g->rhs) != CUFFT_SUCCESS) {
         g->err = "cufftExecZ2D (adjoint)";
@@ -1287,10 +1160,14 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
     }
     k_divT<<<nblk(n), kT, 0, s>>>(P, g->rhs, g->dzf, 1.0, lam_next[0], lam_next[1], lam_next[2]);
     count_launches(1);
-    // 3. z-solve
-    k_zsolve_T<<<nblk(3 * plane), kT, 0, s>>>(P, g->dzc, g->dzf, dt_eff, lam_next[0], lam_next[1],
-                                               lam_next[2], w->scratch);
-    count_launches(1);
+    // 3. z-solve: A^T x = d per column, the forward's kernel with the tables of
+    // the transposed systems
+    double *tab_w = w->zs_tab + zsolve_table_doubles(P.nz) / 2;
+    if (w->zs_dt != dt_eff) {
+        ADJ_CK(launch_zsolve_tables(P, g->dzc, g->dzf, dt_eff, w->zs_tab, tab_w, s, true), "z-solve adjoint tables");
+        w->zs_dt = dt_eff;
+    }
+    ADJ_CK(launch_zsolve(P, TriMut{lam_next[0], lam_next[1], lam_next[2]}, w->zs_tab, tab_w, s), "z-solve adjoint");
     ADJ_CK(cudaGetLastError(), "projection / z-solve adjoint");
     // 4. SL predictor: U* recomputed
     V3 M;

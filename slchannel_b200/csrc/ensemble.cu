@@ -206,12 +206,13 @@ void build_items(slc_ensemble *e, std::vector<EnsItem> &items)
     }
     end(e->r_div);
     e->r_pr = e->r_div;
-    // Poisson Thomas sweep: 4 threads per (kx, ky) column, 256 per block
+    // Poisson Thomas sweep: 4 threads per (kx, ky) column
     begin(e->r_th);
     for (int i = 0; i < n; ++i) {
         const SlcParams &P = e->grids[i]->P;
         const long long nthr = 4LL * P.nx * (P.ny / 2 + 1);
-        const int nb = (int)((nthr + 255) / 256);
+        const int W = thomas_ens_threads();
+        const int nb = (int)((nthr + W - 1) / W);
         for (int b = 0; b < nb; ++b) items.push_back({i, b, 0, 0});
     }
     end(e->r_th);
@@ -273,6 +274,8 @@ int enqueue_step(slc_ensemble *e, int ph, cudaStream_t s)
     const int n = (int)e->grids.size();
     const int cur = ens_cur(ph), nxt = ens_next(ph);
     const EnsInst *I = e->d_inst;
+    int nz_max = 0;
+    for (const slc_grid *g : e->grids) nz_max = std::max(nz_max, g->P.nz);
     ENS_CK(launch_bc_ens(I, items_at(e, e->r_bc), e->r_bc.n, cur, 0, s), "boundary conditions");
     if (e->mixed)
         ENS_CK(launch_mixed_prepare_ens(I, n, items_at(e, e->r_pp), e->r_pp.n, items_at(e, e->r_pack),
@@ -318,7 +321,7 @@ int enqueue_step(slc_ensemble *e, int ph, cudaStream_t s)
         ENS_FFT(cufftSetStream(gr.fwd, s), "cufftSetStream");
         ENS_FFT(cufftExecD2Z(gr.fwd, gr.rhs, (cufftDoubleComplex *)gr.hat), "cufftExecD2Z");
     }
-    ENS_CK(launch_thomas_ens(I, items_at(e, e->r_th), e->r_th.n, s), "Poisson Thomas sweep");
+    ENS_CK(launch_thomas_ens(I, items_at(e, e->r_th), e->r_th.n, nz_max, s), "Poisson Thomas sweep");
     for (auto &gr : e->groups) {
         ENS_FFT(cufftSetStream(gr.inv, s), "cufftSetStream");
         ENS_FFT(cufftExecZ2D(gr.inv, (cufftDoubleComplex *)gr.hat, gr.rhs), "cufftExecZ2D");
@@ -497,7 +500,8 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
         const slc_ensemble::Group &gr = e->groups[group_of[i]];
         I.rhs = gr.rhs + (size_t)plane_off[i] * P.nx * P.ny;
         I.hat = gr.hat + (size_t)2 * plane_off[i] * P.nx * (P.ny / 2 + 1);
-        I.cpw = g->cpw;
+        I.th_id = g->th_id;
+        I.th_g = g->th_g;
         double *tab = nullptr;
         int rc = ealloc(e, &tab, zsolve_table_doubles(P.nz), "z-solve tables");
         if (rc) return rc;

@@ -159,103 +159,175 @@ __global__ void k_divergence(SlcParams P, const double *__restrict__ u,
 
 constexpr int kPre = 8;  // loads kept in flight per thread in the sweeps
 
-// Row k of the (kx, ky) column's system: sub-diagonal a, diagonal b,
-// super-diagonal c (projection.py:47-114), Neumann rows folded into b; the
-// (0, 0) mode's first row is the identity (projection.py:113-114).
+// Row k of the (kx, ky) column's system: sub-diagonal, diagonal and
+// super-diagonal (projection.py:47-114), Neumann rows folded into the diagonal;
+// the (0, 0) mode's first row is the identity (projection.py:113-114).  T: of
+// the transposed system (the adjoint's): the super-diagonal of row k - 1, the
+// diagonal, the sub-diagonal of row k + 1.
+template <bool T>
+__device__ __forceinline__ double poisson_down(const double *__restrict__ cl, const double *__restrict__ cr, int k,
+                                               bool pinned)
+{
+    if (T) return k > 0 && !(pinned && k == 1) ? __ldg(cr + k - 1) : 0.0;
+    return k > 0 ? __ldg(cl + k) : 0.0;
+}
+
+template <bool T>
+__device__ __forceinline__ double poisson_up(const double *__restrict__ cl, const double *__restrict__ cr, int nz,
+                                             int k, bool pinned)
+{
+    if (T) return k < nz - 1 ? __ldg(cl + k + 1) : 0.0;
+    return k < nz - 1 && !(pinned && k == 0) ? __ldg(cr + k) : 0.0;
+}
+
 struct Row3 {
     double a, b, c;
 };
 
-__device__ __forceinline__ Row3 poisson_row(const double *__restrict__ cl,
-                                            const double *__restrict__ cr, double k2, int nz, int k,
-                                            bool pinned)
+template <bool T>
+__device__ __forceinline__ Row3 poisson_row(const double *__restrict__ cl, const double *__restrict__ cr, double k2,
+                                            int nz, int k, bool pinned)
 {
     Row3 r;
-    r.a = k > 0 ? cl[k] : 0.0;
+    r.a = poisson_down<T>(cl, cr, k, pinned);
     r.b = -(cl[k] + cr[k] + k2);
     if (k == 0) r.b += cl[0];
     if (k == nz - 1) r.b += cr[nz - 1];
-    r.c = k < nz - 1 ? cr[k] : 0.0;
-    if (pinned && k == 0) {
-        r.b = 1.0;
-        r.c = 0.0;
-    }
+    if (pinned && k == 0) r.b = 1.0;
+    r.c = poisson_up<T>(cl, cr, nz, k, pinned);
     return r;
 }
 
-// Twisted (two-ended) Thomas elimination: four threads per column, part (re /
-// im) x half.  Half 0 eliminates rows 0 .. m-1 downwards as the reference's
-// Thomas sweep does; half 1 eliminates rows nz-1 .. m+1 upwards (sub- and
-// super-diagonal exchanged); the two meet at row m = nz/2, which the adjacent
-// lanes solve from each other's last pivot row (one shuffle), then each back-
-// substitutes its half.  Twice the threads of a one-ended sweep in flight for
-// the same arithmetic; the meeting row changes results by rounding only.  The
-// coefficients are real, so the real and imaginary parts are independent
-// systems; the part-0 thread of each half stores the pivot ratios g (same
-// values for both parts), read back by both after a warp barrier.
+// Twisted (two-ended) Thomas elimination.  Half 0 eliminates rows 0 .. m-1
+// downwards as the reference's Thomas sweep does; half 1 eliminates rows
+// nz-1 .. m+1 upwards (sub- and super-diagonal exchanged); the two meet at row
+// m = nz/2, and each back-substitutes its half.  The factors depend on the grid
+// alone: k_thomas_factors computes them once per handle (row k of column col at
+// k * ncol + col: th_id the inverse pivots, the meeting row's included, th_g the
+// pivot ratios).  A sweep then has two dependent operations per row where
+// dividing by the pivot on the way was a chain of some thirty: 12.2 -> 6.3 us
+// at 32^3, 24 -> 12 us at 64^3, 211 -> 109 us at 256^3 (0.7 GB: bound there by the
+// traffic, which the table leaves as it was: one word read where a pivot ratio
+// was stored).  The table alone, with the loads of a row still tested one by one
+// behind the chain, was no faster at 64^3 (29 us): the batches below matter as
+// much.
+template <bool T>
+__global__ void __launch_bounds__(256) k_thomas_factors(SlcParams P, double *__restrict__ th_id,
+                                                        double *__restrict__ th_g,
+                                                        const double *__restrict__ kx2,
+                                                        const double *__restrict__ ky2,
+                                                        const double *__restrict__ cl,
+                                                        const double *__restrict__ cr)
+{
+    const int nky = P.ny / 2 + 1;
+    const int ncol = P.nx * nky;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= ncol) return;
+    const int nz = P.nz, m = nz / 2;
+    const int kx = col / nky, ky = col - kx * nky;
+    const double k2 = kx2[kx] + ky2[ky];
+    const bool pinned = col == 0;
+    double gt = 0.0, gb = 0.0;
+    for (int k = 0; k < m; ++k) {
+        const Row3 R = poisson_row<T>(cl, cr, k2, nz, k, pinned);
+        const double id = 1.0 / (R.b - R.a * gt);
+        gt = R.c * id;
+        th_id[(size_t)k * ncol + col] = id;
+        th_g[(size_t)k * ncol + col] = gt;
+    }
+    for (int k = nz - 1; k > m; --k) {
+        const Row3 R = poisson_row<T>(cl, cr, k2, nz, k, pinned);
+        const double id = 1.0 / (R.b - R.c * gb);
+        gb = R.a * id;
+        th_id[(size_t)k * ncol + col] = id;
+        th_g[(size_t)k * ncol + col] = gb;
+    }
+    const Row3 R = poisson_row<T>(cl, cr, k2, nz, m, pinned);
+    th_id[(size_t)m * ncol + col] = 1.0 / (R.b - R.a * gt - R.c * gb);
+    th_g[(size_t)m * ncol + col] = 0.0;
+}
+
+// The sweep: four threads per column, part (re / im) x half, the halves of a
+// part on adjacent lanes (one shuffle joins them at the meeting row); the
+// inverse-FFT normalisation is folded into the back substitution.  Rows go in
+// batches of kPre whose loads are issued one batch ahead without a branch
+// between them (indices are clamped, not tested), so that a row waits for
+// memory once per batch; the couplings to the neighbouring rows come from
+// shared memory (coef: nz sub-, then nz super-diagonals).
+template <bool T>
+__device__ __forceinline__ void thomas_coef(const SlcParams &P, const double *__restrict__ cl,
+                                            const double *__restrict__ cr, double *coef)
+{
+    for (int k = threadIdx.x; k < P.nz; k += blockDim.x) {
+        coef[k] = poisson_down<T>(cl, cr, k, false);
+        coef[P.nz + k] = poisson_up<T>(cl, cr, P.nz, k, false);
+    }
+    __syncthreads();
+}
+
+template <bool T = false>
 __device__ __forceinline__ void thomas_column(const SlcParams &P, double *__restrict__ hat,
-                                              double *__restrict__ cpw,
-                                              const double *__restrict__ kx2,
-                                              const double *__restrict__ ky2,
-                                              const double *__restrict__ cl,
-                                              const double *__restrict__ cr, double norm, int t)
+                                              const double *__restrict__ th_id,
+                                              const double *__restrict__ th_g, const double *coef, double norm,
+                                              int t)
 {
     const int nky = P.ny / 2 + 1;
     const int ncol = P.nx * nky;
     const int col = t >> 2, part = (t >> 1) & 1, half = t & 1;
     const bool active = col < ncol;
     const int nz = P.nz, m = nz / 2;
-    const size_t st = 2 * (size_t)ncol;  // doubles per k-plane of the spectrum
+    const size_t st = 2 * (size_t)ncol, sf = (size_t)ncol;  // doubles per k-plane: spectrum, factors
     double *h = hat + 2 * (size_t)(active ? col : 0) + part;
-    double *cpc = cpw + (active ? col : 0);
-    double k2 = 0.0;
-    if (active) {
-        const int kx = col / nky, ky = col - (col / nky) * nky;
-        k2 = kx2[kx] + ky2[ky];
-    }
-    const bool pinned = active && col == 0;
+    const double *id = th_id + (active ? col : 0), *g = th_g + (active ? col : 0);
     const int cnt = active ? (half ? nz - 1 - m : m) : 0;  // rows this thread eliminates
+    const int last = max(cnt - 1, 0);
+    // the pinned mode's row 0 (transposed: row 1) lacks one coupling
+    const int cut = active && col == 0 ? (T ? 1 : 0) : -1;
+    auto down = [&](int k) { return T && k == cut ? 0.0 : coef[k]; };
+    auto up = [&](int k) { return !T && k == cut ? 0.0 : coef[nz + k]; };
     // row of elimination step q: downwards from 0, or upwards from nz-1
-#define TH_ROW(q) (half ? nz - 1 - (q) : (q))
-    double buf[kPre];
+    auto row = [&](int q) { return half ? nz - 1 - q : q; };
+    double d[kPre], f[kPre], dn[kPre], fn[kPre];
 #pragma unroll
-    for (int q = 0; q < kPre; ++q) buf[q] = q < cnt ? h[TH_ROW(q) * st] : 0.0;
-    double gprev = 0.0, dprev = 0.0;
+    for (int u = 0; u < kPre; ++u) {
+        const int k = row(min(u, last));
+        dn[u] = h[k * st];
+        fn[u] = __ldg(id + k * sf);
+    }
+    double dprev = 0.0;
     for (int q0 = 0; q0 < cnt; q0 += kPre) {
 #pragma unroll
         for (int u = 0; u < kPre; ++u) {
-            const int q = q0 + u;
+            d[u] = dn[u];
+            f[u] = fn[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kPre; ++u) {
+            const int k = row(min(q0 + kPre + u, last));
+            dn[u] = h[k * st];
+            fn[u] = __ldg(id + k * sf);
+        }
+#pragma unroll
+        for (int u = 0; u < kPre; ++u) {
+            const int q = q0 + u, k = row(min(q, last));
+            const double x = (d[u] - (half ? up(k) : down(k)) * dprev) * f[u];
             if (q < cnt) {
-                const int k = TH_ROW(q);
-                const double d = buf[u];
-                if (q + kPre < cnt) buf[u] = h[TH_ROW(q + kPre) * st];
-                const Row3 R = poisson_row(cl, cr, k2, nz, k, pinned);
-                const double e = half ? R.c : R.a, f = half ? R.a : R.c;
-                const double id = 1.0 / (R.b - e * gprev);
-                gprev = f * id;
-                dprev = (d - e * dprev) * id;
-                h[k * st] = dprev;
-                if (part == 0) cpc[k * (size_t)ncol] = gprev;
+                dprev = x;
+                h[k * st] = x;
             }
         }
     }
-#undef TH_ROW
-    // the meeting row m from both halves' last pivot rows
-    const double og = __shfl_xor_sync(0xffffffffu, gprev, 1);
+    // the meeting row m from both halves' last eliminated values
     const double od = __shfl_xor_sync(0xffffffffu, dprev, 1);
-    __syncwarp();  // the pivot ratios stored above are visible to the whole warp
-    const double gt = half ? og : gprev, dtp = half ? od : dprev;  // row m-1 (top)
-    const double gb = half ? gprev : og, dbt = half ? dprev : od;  // row m+1 (bottom)
-    const Row3 R = poisson_row(cl, cr, k2, nz, m, pinned);
-    const double dm = active ? h[m * st] : 0.0;
-    const double xm = (dm - R.a * dtp - R.c * dbt) / (R.b - R.a * gt - R.c * gb);
-    // back substitution outwards from m, prefetching d and g
-    double cb[kPre];
+    const double dtp = half ? od : dprev, dbt = half ? dprev : od;  // rows m-1, m+1
+    const double xm = (h[m * st] - down(m) * dtp - up(m) * dbt) * __ldg(id + m * sf);
+    // back substitution outwards from m
+    auto back = [&](int q) { return half ? min(m + 1 + q, nz - 1) : max(m - 1 - q, 0); };
 #pragma unroll
-    for (int q = 0; q < kPre; ++q) {
-        const int k = half ? m + 1 + q : m - 1 - q;
-        buf[q] = q < cnt ? h[k * st] : 0.0;
-        cb[q] = q < cnt ? cpc[k * (size_t)ncol] : 0.0;
+    for (int u = 0; u < kPre; ++u) {
+        const int k = back(min(u, last));
+        dn[u] = h[k * st];
+        fn[u] = __ldg(g + k * sf);
     }
     __syncwarp();  // every lane has read row m before the top half writes it
     if (active && half == 0) h[m * st] = xm * norm;
@@ -263,30 +335,36 @@ __device__ __forceinline__ void thomas_column(const SlcParams &P, double *__rest
     for (int q0 = 0; q0 < cnt; q0 += kPre) {
 #pragma unroll
         for (int u = 0; u < kPre; ++u) {
+            d[u] = dn[u];
+            f[u] = fn[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kPre; ++u) {
+            const int k = back(min(q0 + kPre + u, last));
+            dn[u] = h[k * st];
+            fn[u] = __ldg(g + k * sf);
+        }
+#pragma unroll
+        for (int u = 0; u < kPre; ++u) {
             const int q = q0 + u;
-            if (q < cnt) {
-                const int k = half ? m + 1 + q : m - 1 - q;
-                const double dk = buf[u], gk = cb[u];
-                if (q + kPre < cnt) {
-                    const int kn = half ? k + kPre : k - kPre;
-                    buf[u] = h[kn * st];
-                    cb[u] = cpc[kn * (size_t)ncol];
-                }
-                x = dk - gk * x;
-                h[k * st] = x * norm;
-            }
+            x = d[u] - f[u] * x;
+            if (q < cnt) h[back(q) * st] = x * norm;
         }
     }
 }
 
-__global__ void __launch_bounds__(256) k_thomas(SlcParams P, double *__restrict__ hat,
-                                                double *__restrict__ cpw,
-                                                const double *__restrict__ kx2,
-                                                const double *__restrict__ ky2,
-                                                const double *__restrict__ cl,
-                                                const double *__restrict__ cr, double norm)
+constexpr int kThomasT = 64;  // small blocks: a 64^3 spectrum's columns still reach most SMs
+
+template <bool T>
+__global__ void __launch_bounds__(kThomasT) k_thomas(SlcParams P, double *__restrict__ hat,
+                                                     const double *__restrict__ th_id,
+                                                     const double *__restrict__ th_g,
+                                                     const double *__restrict__ cl,
+                                                     const double *__restrict__ cr, double norm)
 {
-    thomas_column(P, hat, cpw, kx2, ky2, cl, cr, norm, blockIdx.x * blockDim.x + threadIdx.x);
+    extern __shared__ double coef[];
+    thomas_coef<T>(P, cl, cr, coef);
+    thomas_column<T>(P, hat, th_id, th_g, coef, norm, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // --------------------------------------------------------------------------
@@ -506,13 +584,15 @@ __global__ void __launch_bounds__(256) k_div_pack_ens(const EnsInst *__restrict_
                   I.rhs, it.a, it.b, it.c);
 }
 
-__global__ void __launch_bounds__(256) k_thomas_ens(const EnsInst *__restrict__ ins,
+__global__ void __launch_bounds__(kThomasT) k_thomas_ens(const EnsInst *__restrict__ ins,
                                                     const EnsItem *__restrict__ items)
 {
     const EnsItem it = items[blockIdx.x];
     const EnsInst &I = ins[it.inst];
     const double norm = 1.0 / ((double)I.P.nx * (double)I.P.ny);
-    thomas_column(I.P, I.hat, I.cpw, I.kx2, I.ky2, I.cl, I.cr, norm,
+    extern __shared__ double coef[];
+    thomas_coef<false>(I.P, I.cl, I.cr, coef);
+    thomas_column(I.P, I.hat, I.th_id, I.th_g, coef, norm,
                   it.a * blockDim.x + threadIdx.x);
 }
 
@@ -611,13 +691,26 @@ cudaError_t launch_divergence(const SlcParams &P, Tri f, const double *dz_f, dou
     return cudaGetLastError();
 }
 
-cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, double *cp, const double *kx2,
-                                  const double *ky2, const double *cl, const double *cr,
+cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, double *th_g, const double *kx2,
+                                  const double *ky2, const double *cl, const double *cr, bool transposed,
                                   cudaStream_t s)
+{
+    const unsigned nb = (unsigned)(((long long)P.nx * (P.ny / 2 + 1) + 255) / 256);
+    if (transposed) k_thomas_factors<true><<<nb, 256, 0, s>>>(P, th_id, th_g, kx2, ky2, cl, cr);
+    else k_thomas_factors<false><<<nb, 256, 0, s>>>(P, th_id, th_g, kx2, ky2, cl, cr);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *th_g,
+                                  const double *cl, const double *cr, cudaStream_t s, bool transposed)
 {
     const long long nthr = 4LL * P.nx * (P.ny / 2 + 1);  // thomas_column: 4 per column
     const double norm = 1.0 / ((double)P.nx * (double)P.ny);
-    k_thomas<<<(unsigned)((nthr + 255) / 256), 256, 0, s>>>(P, hat, cp, kx2, ky2, cl, cr, norm);
+    const unsigned nb = (unsigned)((nthr + kThomasT - 1) / kThomasT);
+    const size_t sm = 2 * (size_t)P.nz * sizeof(double);  // nz <= 1024
+    if (transposed) k_thomas<true><<<nb, kThomasT, sm, s>>>(P, hat, th_id, th_g, cl, cr, norm);
+    else k_thomas<false><<<nb, kThomasT, sm, s>>>(P, hat, th_id, th_g, cl, cr, norm);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -668,10 +761,12 @@ cudaError_t launch_div_pack_ens(const EnsInst *ins, const EnsItem *items, int ni
     return cudaGetLastError();
 }
 
-cudaError_t launch_thomas_ens(const EnsInst *ins, const EnsItem *items, int nitems, cudaStream_t s)
+int thomas_ens_threads() { return kThomasT; }
+
+cudaError_t launch_thomas_ens(const EnsInst *ins, const EnsItem *items, int nitems, int nz_max, cudaStream_t s)
 {
     if (nitems <= 0) return cudaSuccess;
-    k_thomas_ens<<<nitems, 256, 0, s>>>(ins, items);
+    k_thomas_ens<<<nitems, kThomasT, 2 * (size_t)nz_max * sizeof(double), s>>>(ins, items);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -173,7 +173,7 @@ int do_project(slc_grid *g, double *u, double *v, double *w, double *p, double d
     SLC_CK(launch_div_pack(g->P, Tri{u, v, w}, g->dzf, dt_div, g->rhs, s), "divergence");
     SLC_FFT(cufftSetStream(g->fwd, s), "cufftSetStream");
     SLC_FFT(cufftExecD2Z(g->fwd, g->rhs, (cufftDoubleComplex *)g->hat), "cufftExecD2Z");
-    SLC_CK(launch_thomas_poisson(g->P, g->hat, g->cpw, g->kx2, g->ky2, g->cl, g->cr, s),
+    SLC_CK(launch_thomas_poisson(g->P, g->hat, g->th_id, g->th_g, g->cl, g->cr, s),
            "Poisson Thomas sweep");
     SLC_FFT(cufftSetStream(g->inv, s), "cufftSetStream");
     SLC_FFT(cufftExecZ2D(g->inv, (cufftDoubleComplex *)g->hat, g->rhs), "cufftExecZ2D");
@@ -702,7 +702,17 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     const size_t nreal = (size_t)nz * nx * ny, ncplx = (size_t)nz * nx * nky;
     CREATE_CK(dalloc(g, &g->rhs, nreal, "Poisson rhs"));
     CREATE_CK(dalloc(g, &g->hat, 2 * ncplx, "Poisson spectrum"));
-    CREATE_CK(dalloc(g, &g->cpw, ncplx, "Poisson Thomas scratch"));
+    CREATE_CK(dalloc(g, &g->th_id, ncplx, "Poisson elimination factors"));
+    CREATE_CK(dalloc(g, &g->th_g, ncplx, "Poisson elimination factors"));
+    {
+        // creation is synchronous: later work may come on any stream
+        cudaError_t e = launch_thomas_factors(P, g->th_id, g->th_g, g->kx2, g->ky2, g->cl, g->cr, false, 0);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        if (e != cudaSuccess) {
+            slc_grid_destroy(g);
+            return fail(nullptr, SLC_E_CUDA, std::string("Poisson elimination factors: ") + cudaGetErrorString(e));
+        }
+    }
     CREATE_CK(dalloc(g, &g->zs_tab, zsolve_table_doubles(nz), "z-solve tables"));
     CREATE_CK(dalloc(g, &g->partials, (size_t)kBulkBlocks, "bulk partials"));
     CREATE_CK(dalloc(g, &g->scal, (size_t)8, "scalars"));

@@ -37,7 +37,7 @@ struct slc_grid {
     float *zc32 = nullptr, *zf32 = nullptr;
     float *dinv_c32[SLC_MAX_ORDER + 1] = {}, *dinv_f32[SLC_MAX_ORDER + 1] = {};
     double *kx2 = nullptr, *ky2 = nullptr, *cl = nullptr, *cr = nullptr;
-    double *rhs = nullptr, *hat = nullptr, *cpw = nullptr;
+    double *rhs = nullptr, *hat = nullptr, *th_id = nullptr, *th_g = nullptr;
     double *zs_tab = nullptr;
     double zs_dt = 0.0;
     bool zs_valid = false;

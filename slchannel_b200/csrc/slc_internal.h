@@ -61,7 +61,8 @@ __host__ __device__ inline int zsolve_chunk(int nz)
 }
 inline size_t zsolve_table_doubles(int nz) { return (size_t)6 * 32 * zsolve_chunk(nz); }
 cudaError_t launch_zsolve_tables(const SlcParams &P, const double *dz_c, const double *dz_f,
-                                 double dt, double *tab_uv, double *tab_w, cudaStream_t s);
+                                 double dt, double *tab_uv, double *tab_w, cudaStream_t s,
+                                 bool transposed = false);
 cudaError_t launch_zsolve(const SlcParams &P, TriMut f, const double *tab_uv, const double *tab_w,
                           cudaStream_t s);
 
@@ -72,9 +73,13 @@ cudaError_t launch_div_pack(const SlcParams &P, Tri f, const double *dz_f, doubl
                             double *rhs_zmajor, cudaStream_t s);
 cudaError_t launch_divergence(const SlcParams &P, Tri f, const double *dz_f, double *div,
                               cudaStream_t s);
-cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, double *cp, const double *kx2,
-                                  const double *ky2, const double *cl, const double *cr,
+// Elimination factors of every (kx, ky) column's z system (or of the
+// transposed systems): two arrays of nz nx (ny/2+1) doubles; and the sweep.
+cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, double *th_g, const double *kx2,
+                                  const double *ky2, const double *cl, const double *cr, bool transposed,
                                   cudaStream_t s);
+cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *th_g,
+                                  const double *cl, const double *cr, cudaStream_t s, bool transposed = false);
 cudaError_t launch_project(const SlcParams &P, const double *phi_zmajor, TriMut f, double *p,
                            const double *dz_c, double dt, cudaStream_t s);
 // bulk: partial sums of u*dz_f over the interior (shift c added first when
@@ -128,7 +133,8 @@ struct EnsInst {
     double *p;
     double *mid[3];                 // U* = 2 V^n - V^{n-1}, ghost-shaped
     const double *dzf, *dzc, *kx2, *ky2, *cl, *cr;
-    double *rhs, *hat, *cpw;        // Poisson workspaces (rhs, hat inside a group's FFT pools)
+    double *rhs, *hat;              // Poisson workspaces (inside a group's FFT pools)
+    const double *th_id, *th_g;     // Poisson elimination factors
     const double *zs_uv, *zs_w;     // z-solve tables at dt_eff = 2 dt / 3
     double *partials, *scal;        // kBulkBlocks partial sums; [shift, forcing]
     unsigned long long *ncl;        // departure-clamp counter
@@ -167,7 +173,8 @@ cudaError_t launch_bc_ens(const EnsInst *ins, const EnsItem *items, int nitems, 
                           int with_p, cudaStream_t s);
 cudaError_t launch_div_pack_ens(const EnsInst *ins, const EnsItem *items, int nitems, int lvl,
                                 cudaStream_t s);
-cudaError_t launch_thomas_ens(const EnsInst *ins, const EnsItem *items, int nitems,
+int thomas_ens_threads();  // threads per work item; nz_max: the largest instance's nz
+cudaError_t launch_thomas_ens(const EnsInst *ins, const EnsItem *items, int nitems, int nz_max,
                               cudaStream_t s);
 cudaError_t launch_project_ens(const EnsInst *ins, const EnsItem *items, int nitems, int lvl,
                                cudaStream_t s);

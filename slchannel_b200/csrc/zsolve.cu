@@ -18,7 +18,10 @@
 
 namespace {
 
-// One thread per system (0: u/v, 1: w); sequential factorisation.
+// One thread per system (0: u/v, 1: w); sequential factorisation.  T: of the
+// transposed systems (row k: the super-diagonal of row k - 1, the diagonal,
+// the sub-diagonal of row k + 1), for the adjoint.
+template <bool T>
 __global__ void k_zsolve_tables(SlcParams P, const double *dz_c, const double *dz_f, double dt,
                                 double *tab_uv, double *tab_w)
 {
@@ -32,8 +35,7 @@ __global__ void k_zsolve_tables(SlcParams P, const double *dz_c, const double *d
     double *al = which == 0 ? tab_uv : tab_w;
     double *inv = al + L;
     double *cp = inv + L;
-    double cprev = 0.0;
-    for (int k = 0; k < n; ++k) {
+    auto row = [&](int k, double &a, double &b, double &c) {
         double dl, dr, dc;
         if (which == 0) {
             dl = dz_c[k];
@@ -47,7 +49,9 @@ __global__ void k_zsolve_tables(SlcParams P, const double *dz_c, const double *d
         const double lower = -alpha / (dl * dc);
         const double center = 1.0 + alpha * (1.0 / dl + 1.0 / dr) / dc;
         const double upper = -alpha / (dr * dc);
-        double a = lower, b = center, c = upper;
+        a = lower;
+        b = center;
+        c = upper;
         if (k == 0) {
             a = 0.0;
             if (which == 0) b = center - lower;  // u[0] = -u[1]
@@ -55,6 +59,22 @@ __global__ void k_zsolve_tables(SlcParams P, const double *dz_c, const double *d
         if (k == n - 1) {
             c = 0.0;
             if (which == 0) b = P.top_neumann ? center + upper : center - upper;
+        }
+    };
+    double cprev = 0.0;
+    double a_up = 0.0, b_up = 0.0, c_up = 0.0, c_down = 0.0;  // T: row k + 1; row k - 1's super-diagonal
+    for (int k = 0; k < n; ++k) {
+        double a, b, c;
+        if (!T) {
+            row(k, a, b, c);
+        } else {
+            if (k == 0) row(0, a_up, b_up, c_up);
+            a = c_down;
+            b = b_up;
+            c_down = c_up;
+            a_up = 0.0;
+            if (k + 1 < n) row(k + 1, a_up, b_up, c_up);
+            c = a_up;
         }
         const double denom = b - a * cprev;
         const double id = 1.0 / denom;
@@ -212,9 +232,10 @@ __global__ void __launch_bounds__(kZWarps * 32) k_zsolve_ens(const EnsInst *__re
 }  // namespace
 
 cudaError_t launch_zsolve_tables(const SlcParams &P, const double *dz_c, const double *dz_f,
-                                 double dt, double *tab_uv, double *tab_w, cudaStream_t s)
+                                 double dt, double *tab_uv, double *tab_w, cudaStream_t s, bool transposed)
 {
-    k_zsolve_tables<<<1, 32, 0, s>>>(P, dz_c, dz_f, dt, tab_uv, tab_w);
+    if (transposed) k_zsolve_tables<true><<<1, 32, 0, s>>>(P, dz_c, dz_f, dt, tab_uv, tab_w);
+    else k_zsolve_tables<false><<<1, 32, 0, s>>>(P, dz_c, dz_f, dt, tab_uv, tab_w);
     count_launches(1);
     return cudaGetLastError();
 }
