@@ -29,6 +29,7 @@
 //    explicit x, y diffusion is the periodic 5-point Laplacian, self-adjoint.
 #include <cufft.h>
 
+#include <algorithm>
 #include <string>
 
 #include "slc_grid.h"
@@ -163,6 +164,7 @@ __device__ void grad_interp(const SlcParams &P, NodeView<double> F, double x, do
     for (int i = 0; i < O; ++i) {
         const int xo = wrap6(b.bx0 + i, P.nx) * F.sx;
         double sy_w = 0.0, sy_dw = 0.0, sy_wz = 0.0;
+#pragma unroll
         for (int j = 0; j < O; ++j) {
             const double *row = F.p + xo + wrap6(b.by0 + j, P.ny) * F.sy + b.k0;
             double s = 0.0, sd = 0.0;
@@ -239,12 +241,12 @@ __device__ __forceinline__ double tri_value_grad(const SlcParams &P, NodeView<do
     return wx0 * r0 + q.tx * r1;
 }
 
-// Trajectory velocity samples (values and gradients) at one point.
+// Trajectory velocity samples (values and gradients) at one point, and the
+// samples' stencils.
 __device__ __forceinline__ void sample3_grad(const SlcParams &P, const V3 &M, double x, double y,
-                                             double z, double (&s)[3], double (&g)[3][3])
+                                             double z, double (&s)[3], double (&g)[3][3], TriShared &t)
 {
     const double zc = clampz(P, z);
-    TriShared t;
     tri_shared(P, x, y, zc, half_cell(P, zc), t);
     const NodeView<double> F[3] = {M.u, M.v, M.w};
 #pragma unroll
@@ -273,7 +275,8 @@ __device__ __forceinline__ void trace_forward(const SlcParams &P, const V3 &M, c
     T.zcl[0] = zr < P.z_lo || zr > P.z_hi;
     for (int it = 1; it < P.n_iters; ++it) {
         double s[3], g[3][3];
-        sample3_grad(P, M, T.m[it - 1][0], T.m[it - 1][1], T.m[it - 1][2], s, g);
+        TriShared t;
+        sample3_grad(P, M, T.m[it - 1][0], T.m[it - 1][1], T.m[it - 1][2], s, g, t);
         zr = a[2] - h * s[2];
         T.m[it][0] = a[0] - h * s[0];
         T.m[it][1] = a[1] - h * s[1];
@@ -285,14 +288,30 @@ __device__ __forceinline__ void trace_forward(const SlcParams &P, const V3 &M, c
     for (int c = 0; c < 3; ++c) T.d[c] = 2.0 * T.m[n][c] - a[c];
 }
 
-// Records of one trilinear sample: position (z clamped) and three coefficients.
-struct TriRec {
-    double x, y, z, cu, cv, cw;
+// The records of the trilinear samples, per field c of U*: key = base node
+// (i0 * ny + j0) * NZ + k0, payload (tx, ty, wz1, coefficient).  Written where
+// the sample's stencils are at hand, one array per field, so that the
+// transposes sort and read nothing else.
+struct TriOut {
+    int *key[3];
+    double4 *pay[3];
 };
+
+__device__ __forceinline__ void write_records(const SlcParams &P, const TriShared &t, const double coef[3],
+                                              const TriOut &out, long long r)
+{
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const TriPiece q = tri_piece(P, c, t);
+        const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
+        out.key[c][r] = (q.i0 * P.ny + q.j0) * NZ + q.k0;
+        out.pay[c][r] = make_double4(q.tx, q.ty, q.wz1, coef[c]);
+    }
+}
 
 __device__ __forceinline__ void trace_backward(const SlcParams &P, const V3 &M, const FootTrace &T,
                                                double h, const double gbar[3], double s0bar[3],
-                                               TriRec *out, long long slot_stride)
+                                               const TriOut &out, long long r0, long long slot_stride)
 {
     const int n = P.n_iters - 1;
     double mb[3] = {2.0 * gbar[0], 2.0 * gbar[1], 2.0 * gbar[2]};
@@ -301,15 +320,9 @@ __device__ __forceinline__ void trace_backward(const SlcParams &P, const V3 &M, 
         // m[it] = a - h S(m[it-1]):  sbar = -h mbar
         const double sb[3] = {-h * mb[0], -h * mb[1], -h * mb[2]};
         double s[3], g[3][3];
-        sample3_grad(P, M, T.m[it - 1][0], T.m[it - 1][1], T.m[it - 1][2], s, g);
-        TriRec r;
-        r.x = T.m[it - 1][0];
-        r.y = T.m[it - 1][1];
-        r.z = T.m[it - 1][2];
-        r.cu = sb[0];
-        r.cv = sb[1];
-        r.cw = sb[2];
-        out[(long long)(it - 1) * slot_stride] = r;
+        TriShared t;
+        sample3_grad(P, M, T.m[it - 1][0], T.m[it - 1][1], T.m[it - 1][2], s, g, t);
+        write_records(P, t, sb, out, r0 + (long long)(it - 1) * slot_stride);
         double nb[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) nb[q] = sb[0] * g[0][q] + sb[1] * g[1][q] + sb[2] * g[2][q];
@@ -333,7 +346,7 @@ __global__ void __launch_bounds__(kT) k_sl_adj_points(SlcParams P, V3 M, const d
                                                       const double *__restrict__ lam_hat, double dt,
                                                       double4 *__restrict__ rec_near,
                                                       double4 *__restrict__ rec_far,
-                                                      TriRec *__restrict__ tri, long long pbase,
+                                                      const __grid_constant__ TriOut tri, long long pbase,
                                                       long long ntot)
 {
     const int nzi = (C == 2) ? P.nz - 1 : P.nz;
@@ -363,7 +376,7 @@ __global__ void __launch_bounds__(kT) k_sl_adj_points(SlcParams P, V3 M, const d
         grad_interp<C, O>(P, ghost_view<double>(C, fn, P.nx, P.ny, P.nz), T.d[0], T.d[1], zdc, gx, gy, gz);
         if (zd < P.z_lo || zd > P.z_hi) gz = 0.0;
         const double gbar[3] = {coef * gx, coef * gy, coef * gz};
-        trace_backward(P, M, T, 0.5 * dt, gbar, s0bar, tri + gp + ntot, ntot);
+        trace_backward(P, M, T, 0.5 * dt, gbar, s0bar, tri, gp + ntot, ntot);
         rec_near[q] = make_double4(T.d[0], T.d[1], zdc, coef);
     }
     if (MODE == 2) {
@@ -377,17 +390,13 @@ __global__ void __launch_bounds__(kT) k_sl_adj_points(SlcParams P, V3 M, const d
                           gz);
         if (zd < P.z_lo || zd > P.z_hi) gz = 0.0;
         const double gbar[3] = {coef * gx, coef * gy, coef * gz};
-        trace_backward(P, M, T, dt, gbar, s0bar, tri + gp + (long long)P.n_iters * ntot, ntot);
+        trace_backward(P, M, T, dt, gbar, s0bar, tri, gp + (long long)P.n_iters * ntot, ntot);
         rec_far[q] = make_double4(T.d[0], T.d[1], zdc, coef);
     }
-    TriRec r;
-    r.x = a[0];
-    r.y = a[1];
-    r.z = a[2];
-    r.cu = s0bar[0];
-    r.cv = s0bar[1];
-    r.cw = s0bar[2];
-    tri[gp] = r;
+    const double za = clampz(P, a[2]);
+    TriShared t;
+    tri_shared(P, a[0], a[1], za, half_cell(P, za), t);
+    write_records(P, t, s0bar, tri, gp);
 }
 
 // ---- records -> (key, payload) -----------------------------------------------
@@ -432,23 +441,6 @@ __global__ void __launch_bounds__(kT) k_sorted_weights(SlcParams P, const double
         W[(size_t)(2 * O + m) * n + p] = wz[m];
     }
     kz[p] = b.k0;
-}
-
-// Trilinear records for field c of U*: payload (tx, ty, wz1, coef_c).
-__global__ void k_tri_keys(SlcParams P, int c, const TriRec *__restrict__ tri, long long n,
-                           int *__restrict__ keys, double4 *__restrict__ pay)
-{
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const TriRec R = tri[r];
-    const double zc = clampz(P, R.z);
-    TriShared t;
-    tri_shared(P, R.x, R.y, zc, half_cell(P, zc), t);
-    const TriPiece q = tri_piece(P, c, t);
-    const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
-    keys[r] = (q.i0 * P.ny + q.j0) * NZ + q.k0;
-    const double coef = c == 0 ? R.cu : (c == 1 ? R.cv : R.cw);
-    pay[r] = make_double4(q.tx, q.ty, q.wz1, coef);
 }
 
 // ---- counting sort by key (integer atomics only; deterministic order) -------
@@ -571,48 +563,86 @@ __global__ void k_sort_segments(const int *__restrict__ starts, long long nkeys,
 }
 
 // ---- pulls: every target node sums the records whose stencil covers it -----
-// For each (mx, my), the stencil starts covering node iz along z are the
-// consecutive keys k0 = iz - O + 1 .. iz, so their records are one contiguous
-// range of the sorted order: two starts loads per (mx, my), then four
-// coalesced loads per record (lanes are consecutive iz, their ranges shifted
-// by one key).  Records are summed in key order, then record id: a fixed
-// order, so the result is reproducible bit for bit.
-#ifndef SLC_PULL_UNROLL
-#define SLC_PULL_UNROLL 2
-#endif
-constexpr int kPullUnroll = SLC_PULL_UNROLL;  // records per trip of the pull's inner loop
+// Two passes, both in a fixed order, so the result is reproducible bit for bit.
+//
+// (1) k_pull_columns: one thread per x base bx, z node iz and segment of y
+// walks the y bases of its segment upwards.  At each base the records that
+// cover iz along z are one contiguous range of the sorted order (the keys
+// iz - O + 1 .. iz); a record's weights are loaded once and serve all O x O
+// (mx, my) nodes it reaches, accumulated in registers: acc[mx][my] belongs to
+// node (bx + mx, by + my).  Moving on to by + 1 completes node row by, whose O
+// sums go to U[mx], and shifts the rest.  A segment starts O - 1 bases early to
+// collect what earlier bases give its first rows.
+// (2) k_pull_rows: node (ix, iy, iz) adds the U[mx] of the O bases ix - mx.
+//
+// A pull by node (each node visiting all O^3 bases that cover it) loads four
+// words for each of its 216 or so records: 672 us per component and foot at
+// 128 x 96 x 128, order 6, bound by the L1 data pipe at 80 %.  Here a record's
+// 2 O + 2 words are loaded once per z node it reaches: 180 us for the first pass
+// (latency of a record's loads at 16 warps an SM), 20 us for the second.
+
 template <int C, int O>
-__global__ void __launch_bounds__(kT) k_pull_gather(SlcParams P, const double *__restrict__ W,
-                                                    const int *__restrict__ kz, long long nrec,
-                                                    const int *__restrict__ starts, double *lam)
+__global__ void __launch_bounds__(kT, 2) k_pull_columns(SlcParams P, const double *__restrict__ W,
+                                                     const int *__restrict__ kz, long long nrec,
+                                                     const int *__restrict__ starts, int nseg, int len,
+                                                     double *__restrict__ U)
+{
+    const int NZ = Comp<C>::centers ? P.nz + 2 : P.nz + 1;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)P.nx * nseg * NZ) return;
+    const int iz = (int)(t % NZ);
+    const int seg = (int)((t / NZ) % nseg);
+    const int bx = (int)(t / ((long long)NZ * nseg));
+    const int y0 = seg * len, y1 = min(y0 + len, P.ny);
+    const int klo = max(iz - (O - 1), 0), khi = min(iz, NZ - O);
+    const size_t nodes = (size_t)P.nx * P.ny * NZ;
+    double acc[O][O];
+#pragma unroll
+    for (int m = 0; m < O; ++m)
+#pragma unroll
+        for (int q = 0; q < O; ++q) acc[m][q] = 0.0;
+    for (int y = y0 - (O - 1); y < y1; ++y) {
+        const int kb = (bx * P.ny + wrap6(y, P.ny)) * NZ;
+        const int a = __ldg(starts + kb + klo), b = __ldg(starts + kb + khi + 1);
+        for (int p = a; p < b; ++p) {
+            const double wz = __ldg(W + (size_t)(2 * O + iz - __ldg(kz + p)) * nrec + p);
+            double wy[O];
+#pragma unroll
+            for (int q = 0; q < O; ++q) wy[q] = __ldg(W + (size_t)(O + q) * nrec + p);
+#pragma unroll
+            for (int m = 0; m < O; ++m) {
+                const double c = __ldg(W + (size_t)m * nrec + p) * wz;
+#pragma unroll
+                for (int q = 0; q < O; ++q) acc[m][q] = fma(c, wy[q], acc[m][q]);
+            }
+        }
+        if (y >= y0) {
+#pragma unroll
+            for (int m = 0; m < O; ++m) U[m * nodes + kb + iz] = acc[m][0];
+        }
+#pragma unroll
+        for (int m = 0; m < O; ++m) {
+#pragma unroll
+            for (int q = 0; q + 1 < O; ++q) acc[m][q] = acc[m][q + 1];
+            acc[m][O - 1] = 0.0;
+        }
+    }
+}
+
+template <int C, int O>
+__global__ void __launch_bounds__(kT) k_pull_rows(SlcParams P, const double *__restrict__ U, double *lam)
 {
     const int NZ = Comp<C>::centers ? P.nz + 2 : P.nz + 1;
     const long long nn = (long long)P.nx * P.ny * NZ;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nn) return;
-    const int iz = (int)(t % NZ);
-    const int iy = (int)((t / NZ) % P.ny);
-    const int ix = (int)(t / ((long long)NZ * P.ny));
-    const int klo = max(iz - (O - 1), 0), khi = min(iz, NZ - O);
+    const long long row = (long long)P.ny * NZ;
+    const int ix = (int)(t / row);
+    const long long r = t - ix * row;
     double acc = 0.0;
-    if (klo <= khi) {
-        for (int mx = 0; mx < O; ++mx) {
-            const int bx = wrap6(ix - mx, P.nx);
-            const double *cwx = W + (size_t)mx * nrec;
-            for (int my = 0; my < O; ++my) {
-                const int by = wrap6(iy - my, P.ny);
-                const double *wyv = W + (size_t)(O + my) * nrec;
-                const int kb = (bx * P.ny + by) * NZ;
-                const int a = __ldg(starts + kb + klo), b = __ldg(starts + kb + khi + 1);
-#pragma unroll kPullUnroll
-                for (int p = a; p < b; ++p) {
-                    const int mz = iz - __ldg(kz + p);
-                    const double wz = __ldg(W + (size_t)(2 * O + mz) * nrec + p);
-                    acc = fma(__ldg(cwx + p) * __ldg(wyv + p), wz, acc);
-                }
-            }
-        }
-    }
+#pragma unroll
+    for (int m = 0; m < O; ++m) acc += __ldg(U + m * nn + wrap6(ix - m, P.nx) * row + r);
+    const int iy = (int)(r / NZ), iz = (int)(r - (long long)iy * NZ);
     const NodeView<double> V = ghost_view<double>(C, lam, P.nx, P.ny, P.nz);
     double *dst = const_cast<double *>(V.p) + (size_t)ix * V.sx + (size_t)iy * V.sy + iz;
     *dst += acc;
@@ -873,8 +903,8 @@ __global__ void k_axpy(double *y, const double *__restrict__ x, double a, long l
 
 struct AdjWS {
     long long n_c[3] = {0, 0, 0}, ntot = 0, nkeys_max = 0, nrec_max = 0;
-    double4 *rec_near = nullptr, *rec_far = nullptr, *pay = nullptr;
-    TriRec *tri = nullptr;
+    double4 *rec_near = nullptr, *rec_far = nullptr;
+    TriOut tri{};
     int *keys = nullptr, *order = nullptr, *counts = nullptr, *starts = nullptr, *fill = nullptr;
     int *sums = nullptr, *total = nullptr;
     double *lam_mid[3] = {nullptr, nullptr, nullptr};
@@ -883,7 +913,9 @@ struct AdjWS {
     double *partials = nullptr, *S = nullptr;
     double *W = nullptr;  // sorted gather weights, 3 O arrays of n_c[0]
     int *kz = nullptr;    // sorted gather records' first z node
-    double *Stri = nullptr;  // trilinear corner partials, 8 arrays of nkeys_max
+    // partial sums over the bases: 8 trilinear corners, or O x offsets of a
+    // gather's transpose (arrays of nkeys_max)
+    double *part = nullptr;
 };
 
 namespace {
@@ -926,9 +958,11 @@ int ensure_adj(slc_grid *g, cudaStream_t s)
     const long long nb = (w->nkeys_max + 1 + kScanT - 1) / kScanT;
     int rc = adj_alloc(g, &w->rec_near, (size_t)w->n_c[0], "adjoint near records");
     if (!rc) rc = adj_alloc(g, &w->rec_far, (size_t)w->n_c[0], "adjoint far records");
-    if (!rc) rc = adj_alloc(g, &w->tri, (size_t)w->nrec_max, "adjoint trajectory records");
-    if (!rc) rc = adj_alloc(g, &w->pay, (size_t)w->nrec_max, "adjoint payload");
-    if (!rc) rc = adj_alloc(g, &w->keys, (size_t)w->nrec_max, "adjoint keys");
+    for (int c = 0; c < 3 && !rc; ++c) {
+        rc = adj_alloc(g, &w->tri.key[c], (size_t)w->nrec_max, "adjoint trajectory keys");
+        if (!rc) rc = adj_alloc(g, &w->tri.pay[c], (size_t)w->nrec_max, "adjoint trajectory records");
+    }
+    if (!rc) rc = adj_alloc(g, &w->keys, (size_t)w->n_c[0], "adjoint keys");
     if (!rc) rc = adj_alloc(g, &w->order, (size_t)w->nrec_max, "adjoint order");
     if (!rc) rc = adj_alloc(g, &w->counts, (size_t)w->nkeys_max + 1, "adjoint counts");
     if (!rc) rc = adj_alloc(g, &w->starts, (size_t)w->nkeys_max + 1, "adjoint starts");
@@ -941,7 +975,7 @@ int ensure_adj(slc_grid *g, cudaStream_t s)
     if (!rc) rc = adj_alloc(g, &w->S, (size_t)1, "adjoint sum");
     if (!rc) rc = adj_alloc(g, &w->W, (size_t)3 * SLC_MAX_ORDER * w->n_c[0], "adjoint gather weights");
     if (!rc) rc = adj_alloc(g, &w->kz, (size_t)w->n_c[0], "adjoint gather z bases");
-    if (!rc) rc = adj_alloc(g, &w->Stri, (size_t)8 * w->nkeys_max, "adjoint trilinear partials");
+    if (!rc) rc = adj_alloc(g, &w->part, (size_t)8 * w->nkeys_max, "adjoint partial sums");
     const size_t ncplx = (size_t)P.nz * P.nx * (P.ny / 2 + 1);
     if (!rc) rc = adj_alloc(g, &w->th_id, ncplx, "adjoint Poisson factors");
     if (!rc) rc = adj_alloc(g, &w->th_g, ncplx, "adjoint Poisson factors");
@@ -959,22 +993,39 @@ int ensure_adj(slc_grid *g, cudaStream_t s)
     return SLC_OK;
 }
 
-// Counting sort of w->keys[0, n) over nkeys keys into w->order / w->starts.
-int sort_records(slc_grid *g, AdjWS *w, long long n, long long nkeys, cudaStream_t s)
+// Counting sort of keys[0, n) over nkeys keys into w->order / w->starts.
+int sort_records(slc_grid *g, AdjWS *w, const int *keys, long long n, long long nkeys, cudaStream_t s)
 {
     k_izero<<<nblk(nkeys + 1), kT, 0, s>>>(w->counts, nkeys + 1);
     k_izero<<<nblk(nkeys + 1), kT, 0, s>>>(w->fill, nkeys + 1);
-    if (n > 0) k_count<<<nblk(n), kT, 0, s>>>(w->keys, n, w->counts);
+    if (n > 0) k_count<<<nblk(n), kT, 0, s>>>(keys, n, w->counts);
     const long long m = nkeys + 1;
     const int nb = (int)((m + kScanT - 1) / kScanT);
     k_scan_blocks<<<nb, kScanT, 0, s>>>(w->counts, w->starts, w->sums, m);
     k_scan_sums<<<1, kScanT, 0, s>>>(w->sums, nb, w->total);
     k_scan_add<<<nb, kScanT, 0, s>>>(w->starts, w->sums, m);
-    if (n > 0) k_place<<<nblk(n), kT, 0, s>>>(w->keys, n, w->starts, w->fill, w->order);
+    if (n > 0) k_place<<<nblk(n), kT, 0, s>>>(keys, n, w->starts, w->fill, w->order);
     k_sort_segments<<<nblk(nkeys), kT, 0, s>>>(w->starts, nkeys, w->order);
     count_launches(n > 0 ? 9 : 7);
     ADJ_CK(cudaGetLastError(), "adjoint record sort");
     return SLC_OK;
+}
+
+// y rows per segment of k_pull_columns: the length with the least waves of
+// blocks (two of 256 threads an SM) times bases walked per segment.
+int pull_segment(const SlcParams &P, int NZ, int O)
+{
+    int best = 8;
+    long long least = -1;
+    for (int len = 8; len <= 64; ++len) {
+        const long long threads = (long long)P.nx * ((P.ny + len - 1) / len) * NZ;
+        const long long cost = ((threads + 148 * 512 - 1) / (148 * 512)) * (std::min(len, P.ny) + O - 1);
+        if (least < 0 || cost < least) {
+            least = cost;
+            best = len;
+        }
+    }
+    return best;
 }
 
 template <int O, int MODE>
@@ -1001,6 +1052,9 @@ int sl_adjoint_t(slc_grid *g, AdjWS *w, const V3 &M, const double *const cur[3],
         count_launches(1);
         const int NZ = C < 2 ? P.nz + 2 : P.nz + 1;
         const long long nkeys = (long long)P.nx * P.ny * NZ;
+        const int seg_len = pull_segment(P, NZ, O);
+        const int nseg = (P.ny + seg_len - 1) / seg_len;
+        const long long ncols = (long long)P.nx * nseg * NZ;
         // near foot -> lam_cur[C]; far foot -> lam_prev[C]
         for (int foot = 0; foot < (MODE == 2 ? 2 : 1); ++foot) {
             const double4 *rec = foot == 0 ? w->rec_near : w->rec_far;
@@ -1009,19 +1063,22 @@ int sl_adjoint_t(slc_grid *g, AdjWS *w, const V3 &M, const double *const cur[3],
             else if (C == 1) k_gather_keys<1, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->keys);
             else k_gather_keys<2, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->keys);
             count_launches(1);
-            int rc = sort_records(g, w, n, nkeys, s);
+            int rc = sort_records(g, w, w->keys, n, nkeys, s);
             if (rc) return rc;
             if (C == 0) {
                 k_sorted_weights<0, O><<<nblk(n), kT, 0, s>>>(P, rec, w->order, n, w->W, w->kz);
-                k_pull_gather<0, O><<<nblk(nkeys), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, dst);
+                k_pull_columns<0, O><<<nblk(ncols), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, nseg, seg_len, w->part);
+                k_pull_rows<0, O><<<nblk(nkeys), kT, 0, s>>>(P, w->part, dst);
             } else if (C == 1) {
                 k_sorted_weights<1, O><<<nblk(n), kT, 0, s>>>(P, rec, w->order, n, w->W, w->kz);
-                k_pull_gather<1, O><<<nblk(nkeys), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, dst);
+                k_pull_columns<1, O><<<nblk(ncols), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, nseg, seg_len, w->part);
+                k_pull_rows<1, O><<<nblk(nkeys), kT, 0, s>>>(P, w->part, dst);
             } else {
                 k_sorted_weights<2, O><<<nblk(n), kT, 0, s>>>(P, rec, w->order, n, w->W, w->kz);
-                k_pull_gather<2, O><<<nblk(nkeys), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, dst);
+                k_pull_columns<2, O><<<nblk(ncols), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, nseg, seg_len, w->part);
+                k_pull_rows<2, O><<<nblk(nkeys), kT, 0, s>>>(P, w->part, dst);
             }
-            count_launches(2);
+            count_launches(3);
         }
         // explicit x, y diffusion
         const double cc = MODE == 2 ? (P.xy_lagged ? (2.0 / 3.0) * dt : (4.0 / 3.0) * dt) : dt;
@@ -1036,14 +1093,12 @@ int sl_adjoint_t(slc_grid *g, AdjWS *w, const V3 &M, const double *const cur[3],
     const long long nrec = (long long)(MODE == 2 ? 2 * P.n_iters - 1 : P.n_iters) * w->ntot;
     for (int c = 0; c < 3; ++c) {
         ADJ_CK(cudaMemsetAsync(w->lam_mid[c], 0, g->ghost_elems[c] * sizeof(double), s), "memset");
-        k_tri_keys<<<nblk(nrec), kT, 0, s>>>(P, c, w->tri, nrec, w->keys, w->pay);
-        count_launches(1);
         const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
         const long long nkeys = (long long)P.nx * P.ny * NZ;
-        int rc = sort_records(g, w, nrec, nkeys, s);
+        int rc = sort_records(g, w, w->tri.key[c], nrec, nkeys, s);
         if (rc) return rc;
-        k_tri_segsum<<<nblk(nkeys), kT, 0, s>>>(w->pay, w->order, w->starts, nkeys, w->Stri);
-        k_pull_tri<<<nblk(nkeys), kT, 0, s>>>(P, c, w->Stri, w->lam_mid[c]);
+        k_tri_segsum<<<nblk(nkeys), kT, 0, s>>>(w->tri.pay[c], w->order, w->starts, nkeys, w->part);
+        k_pull_tri<<<nblk(nkeys), kT, 0, s>>>(P, c, w->part, w->lam_mid[c]);
         count_launches(2);
         // U* = 2 V^n - V^{n-1} (BDF2) or V^n (BDF1)
         const long long ne = (long long)g->ghost_elems[c];
