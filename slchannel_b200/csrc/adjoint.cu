@@ -1234,9 +1234,9 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
                 g->allocs.push_back(q);
                 g->mid[c] = (double *)q;
             }
-        for (int c = 0; c < 3; ++c)
-            ADJ_CK(launch_lincomb(cur[c], prev[c], 2.0, -1.0, g->mid[c], (int64_t)g->ghost_elems[c], s),
-                   "U*");
+        ADJ_CK(launch_star(Tri{cur[0], cur[1], cur[2]}, Tri{prev[0], prev[1], prev[2]},
+                           TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->ghost_elems, s),
+               "U*");
         M.u = ghost_view<double>(0, g->mid[0], P.nx, P.ny, P.nz);
         M.v = ghost_view<double>(1, g->mid[1], P.nx, P.ny, P.nz);
         M.w = ghost_view<double>(2, g->mid[2], P.nx, P.ny, P.nz);

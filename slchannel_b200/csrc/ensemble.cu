@@ -219,7 +219,7 @@ void build_items(slc_ensemble *e, std::vector<EnsItem> &items)
     // bulk partial sums: the single-channel block decomposition per instance
     begin(e->r_bulk);
     for (int i = 0; i < n; ++i)
-        for (int b = 0; b < kBulkBlocks; ++b) items.push_back({i, b, 0, 0});
+        for (int b = 0; b < bulk_blocks(e->grids[i]->P.nx, e->grids[i]->P.ny); ++b) items.push_back({i, b, 0, 0});
     end(e->r_bulk);
     // mixed form: plane-mean partials (column group, field) and FP32 packs
     begin(e->r_pp);

@@ -523,13 +523,13 @@ __global__ void __launch_bounds__(256) k_bulk_partials(SlcParams P, double *__re
     bulk_partial(P, u, dz_f, c_dev, partials, blockIdx.x, gridDim.x);
 }
 
-__device__ __forceinline__ void bulk_finish(const double *__restrict__ partials, int nparts,
+__device__ __forceinline__ void bulk_finish(const double *partials, int nparts,
                                             double dxdy_over_V, double U_bulk, double dt,
                                             double *bulk_out, double *shift_out)
 {
     __shared__ double red[256];
     double acc = 0.0;
-    for (int b = threadIdx.x; b < nparts; b += blockDim.x) acc += partials[b];
+    for (int b = threadIdx.x; b < nparts; b += blockDim.x) acc += __ldcg(partials + b);
     red[threadIdx.x] = acc;
     __syncthreads();
     for (int s = 128; s > 0; s >>= 1) {
@@ -551,6 +551,30 @@ __global__ void k_bulk_finish(const double *__restrict__ partials, int nparts, d
                               double U_bulk, double dt, double *bulk_out, double *shift_out)
 {
     bulk_finish(partials, nparts, dxdy_over_V, U_bulk, dt, bulk_out, shift_out);
+}
+
+// Both in one launch: the last block to store its partial sum adds them up, in
+// k_bulk_finish's order.  *ticket is 0 before and after.  mode 0: shift_out =
+// [U_bulk - bulk, (U_bulk - bulk) / dt]; mode 1 (c_dev = that shift): out2 =
+// [bulk after the shift, c_dev[1]].  A bulk shift is two of these and a ghost
+// refresh instead of six operations: 17.5 -> BS us of a 32^3 step.
+__global__ void __launch_bounds__(256) k_bulk_sum(SlcParams P, double *__restrict__ u,
+                                                  const double *__restrict__ dz_f,
+                                                  const double *c_dev, double *partials, unsigned *ticket,
+                                                  double dxdy_over_V, double U_bulk, double dt, double *bulk_out,
+                                                  double *shift_out)
+{
+    __shared__ bool s_last;
+    bulk_partial(P, u, dz_f, c_dev, partials, blockIdx.x, gridDim.x);
+    if (threadIdx.x == 0) {
+        __threadfence();  // the partial sum is visible before the ticket
+        s_last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    bulk_finish(partials, gridDim.x, dxdy_over_V, U_bulk, dt, bulk_out, shift_out);
+    if (bulk_out && c_dev && threadIdx.x == 0) bulk_out[1] = c_dev[1];
 }
 
 // ---- ensemble forms: one block per item, the instance's own arithmetic ----
@@ -612,7 +636,7 @@ __global__ void __launch_bounds__(256) k_bulk_partials_ens(const EnsInst *__rest
     const EnsItem it = items[blockIdx.x];
     const EnsInst &I = ins[it.inst];
     bulk_partial(I.P, I.lev[lvl][0], I.dzf, with_shift ? I.scal : nullptr, I.partials, it.a,
-                 kBulkBlocks);
+                 bulk_blocks(I.P.nx, I.P.ny));
 }
 
 __global__ void k_bulk_finish_ens(const EnsInst *__restrict__ ins, int mode)
@@ -620,9 +644,9 @@ __global__ void k_bulk_finish_ens(const EnsInst *__restrict__ ins, int mode)
     const EnsInst &I = ins[blockIdx.x];
     const double dxdy_over_V = (I.P.dx * I.P.dy) / (I.Lx * I.Ly * I.P.Lz);
     if (mode == 0) {
-        bulk_finish(I.partials, kBulkBlocks, dxdy_over_V, I.U_bulk, I.dt, nullptr, I.scal);
+        bulk_finish(I.partials, bulk_blocks(I.P.nx, I.P.ny), dxdy_over_V, I.U_bulk, I.dt, nullptr, I.scal);
     } else {
-        bulk_finish(I.partials, kBulkBlocks, dxdy_over_V, 0.0, 1.0, I.bulk_out, nullptr);
+        bulk_finish(I.partials, bulk_blocks(I.P.nx, I.P.ny), dxdy_over_V, 0.0, 1.0, I.bulk_out, nullptr);
         if (threadIdx.x == 0) I.bulk_out[1] = I.scal[1];
     }
 }
@@ -727,7 +751,7 @@ cudaError_t launch_project(const SlcParams &P, const double *phi_zmajor, TriMut 
 cudaError_t launch_bulk_partials(const SlcParams &P, double *u, const double *dz_f,
                                  const double *c_dev, double *partials, cudaStream_t s)
 {
-    k_bulk_partials<<<kBulkBlocks, 256, 0, s>>>(P, u, dz_f, c_dev, partials);
+    k_bulk_partials<<<bulk_blocks(P.nx, P.ny), 256, 0, s>>>(P, u, dz_f, c_dev, partials);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -737,8 +761,19 @@ cudaError_t launch_bulk_finish(const SlcParams &P, const double *partials, doubl
                                cudaStream_t s)
 {
     const double dxdy_over_V = (P.dx * P.dy) / (Lx * Ly * P.Lz);
-    k_bulk_finish<<<1, 256, 0, s>>>(partials, kBulkBlocks, dxdy_over_V, U_bulk, dt, bulk_out,
+    k_bulk_finish<<<1, 256, 0, s>>>(partials, bulk_blocks(P.nx, P.ny), dxdy_over_V, U_bulk, dt, bulk_out,
                                     shift_out);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bulk_sum(const SlcParams &P, double *u, const double *dz_f, const double *c_dev,
+                            double *partials, unsigned *ticket, double Lx, double Ly, double U_bulk, double dt,
+                            double *bulk_out, double *shift_out, cudaStream_t s)
+{
+    const double dxdy_over_V = (P.dx * P.dy) / (Lx * Ly * P.Lz);
+    k_bulk_sum<<<bulk_blocks(P.nx, P.ny), 256, 0, s>>>(P, u, dz_f, c_dev, partials, ticket, dxdy_over_V, U_bulk, dt, bulk_out,
+                                           shift_out);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -345,9 +345,11 @@ __global__ void __launch_bounds__(kThreads, SLC_SLM_MIN_BLOCKS)
     const int k = blockIdx.x * kTileK + (threadIdx.x % kTileK);
     const int j = blockIdx.y * kTileJ + (threadIdx.x / kTileK);
     const int i = blockIdx.z;
+    overlap_begin();
     unsigned ncl = 0;
     sl_point_mixed<C, O, MODE, TO>(P, M, FA, FB, fn, fnm1, dt, out, i, j, k, ncl, om);
     add_clamps(nclamp, ncl);
+    overlap_end();
 }
 
 // ---- the BDF2 trace+gather with TMA-staged FP32 boxes ------------------------
@@ -561,6 +563,7 @@ __global__ void __launch_bounds__(kThreads, SLC_SLMT_MIN_BLOCKS)
     const int nzi = (C == 2) ? P.nz - 1 : P.nz;
     const bool act = k < nzi && j < P.ny && i < P.nx;
     const unsigned barA = smem_u32(&mbar[0]), barB = smem_u32(&mbar[1]);
+    overlap_begin();
     if (tid == 0) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
@@ -646,6 +649,7 @@ __global__ void __launch_bounds__(kThreads, SLC_SLMT_MIN_BLOCKS)
     }
     add_clamps(nclamp, ncl);
     if (tid == 0 && fitB && !mbar_wait(barB)) atomicAdd(stats, 1ull);
+    overlap_end();
 }
 
 // ---- plane means -----------------------------------------------------------
@@ -971,14 +975,13 @@ void launch_tt(const SlcParams &P, Tri fn, Tri fnm1, const MixedWS &ws, double d
     const dim3 gc((P.nz + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
     const dim3 gw((P.nz - 1 + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
     const OutMap ghost{0, 0, 0};
-    k_sl_mixed<0, O, MODE, TO><<<gc, kThreads, 0, s>>>(P, M, mview(ws, 0, P), mview(ws, 3, P), fn.u,
-                                                    fnm1.u, dt, out.u, ncl, om ? om[0] : ghost);
-    k_sl_mixed<1, O, MODE, TO><<<gc, kThreads, 0, s>>>(P, M, mview(ws, 1, P), mview(ws, 4, P), fn.v,
-                                                    fnm1.v, dt, out.v, ncl, om ? om[1] : ghost);
+    launch_chained(k_sl_mixed<0, O, MODE, TO>, gc, kThreads, 0, s, false, P, M, mview(ws, 0, P), mview(ws, 3, P), fn.u,
+                   fnm1.u, dt, out.u, ncl, om ? om[0] : ghost);
+    launch_chained(k_sl_mixed<1, O, MODE, TO>, gc, kThreads, 0, s, true, P, M, mview(ws, 1, P), mview(ws, 4, P), fn.v,
+                   fnm1.v, dt, out.v, ncl, om ? om[1] : ghost);
     if (P.nz > 1)
-        k_sl_mixed<2, O, MODE, TO><<<gw, kThreads, 0, s>>>(P, M, mview(ws, 2, P), mview(ws, 5, P),
-                                                        fn.w, fnm1.w, dt, out.w, ncl,
-                                                        om ? om[2] : ghost);
+        launch_chained(k_sl_mixed<2, O, MODE, TO>, gw, kThreads, 0, s, true, P, M, mview(ws, 2, P), mview(ws, 5, P),
+                       fn.w, fnm1.w, dt, out.w, ncl, om ? om[2] : ghost);
     count_launches(P.nz > 1 ? 3 : 2);
 }
 
@@ -1075,13 +1078,13 @@ cudaError_t launch_mtma_t(const SlcParams &P, const Vel3M &M, const MixedView *F
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_sl_mixed_tma<2, O, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_sl_mixed_tma<0, O, TO><<<gc, kThreads, sm, s>>>(P, M, FA[0], FB[0], fn.u, fnm1.u, dt, out.u, ncl, stats,
-                                                      tm[0], tm[3]);
-    k_sl_mixed_tma<1, O, TO><<<gc, kThreads, sm, s>>>(P, M, FA[1], FB[1], fn.v, fnm1.v, dt, out.v, ncl, stats,
-                                                      tm[1], tm[4]);
+    launch_chained(k_sl_mixed_tma<0, O, TO>, gc, kThreads, sm, s, false, P, M, FA[0], FB[0], fn.u, fnm1.u, dt, out.u, ncl,
+                   stats, tm[0], tm[3]);
+    launch_chained(k_sl_mixed_tma<1, O, TO>, gc, kThreads, sm, s, true, P, M, FA[1], FB[1], fn.v, fnm1.v, dt, out.v, ncl,
+                   stats, tm[1], tm[4]);
     if (P.nz > 1)
-        k_sl_mixed_tma<2, O, TO><<<gw, kThreads, sm, s>>>(P, M, FA[2], FB[2], fn.w, fnm1.w, dt, out.w, ncl,
-                                                          stats, tm[2], tm[5]);
+        launch_chained(k_sl_mixed_tma<2, O, TO>, gw, kThreads, sm, s, true, P, M, FA[2], FB[2], fn.w, fnm1.w, dt, out.w,
+                       ncl, stats, tm[2], tm[5]);
     count_launches(P.nz > 1 ? 3 : 2);
     return cudaGetLastError();
 }

@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, Box<O>::min_blocks)
     const int nzi = (C == 2) ? P.nz - 1 : P.nz;
     const bool act = k < nzi && j < P.ny && i < P.nx;
     const unsigned barN = smem_u32(&mbar[0]), barM = smem_u32(&mbar[1]);
+    overlap_begin();
     if (tid == 0) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
@@ -396,18 +397,21 @@ __global__ void __launch_bounds__(kThreads, Box<O>::min_blocks)
     }
     add_clamps(nclamp, ncl);
     if (tid == 0 && fitM && !mbar_wait(barM)) atomicAdd(stats, 1ull);
+    overlap_end();
 }
+
+__host__ __device__ inline int padded_nz(int NZ) { return (NZ + 1) & ~1; }
 
 // U* = 2 V^n - V^{n-1} at every node (ghost-shaped, node entries only) and
 // the halo-padded node copies of V^n and V^{n-1}.  One warp per padded
 // (x, y) row, lanes along z (contiguous in both layouts); the row's source
 // (x mod nx, y mod ny) is found once per row.
 template <int C>
-__global__ void __launch_bounds__(256) k_mid_pack(SlcParams P, const double *__restrict__ a,
-                                                  const double *__restrict__ b, double ca, double cb,
-                                                  double *__restrict__ mid, double *__restrict__ pa,
-                                                  double *__restrict__ pb, int NZp)
+__device__ __forceinline__ void mid_pack(const SlcParams &P, const double *__restrict__ a,
+                                         const double *__restrict__ b, double *__restrict__ mid,
+                                         double *__restrict__ pa, double *__restrict__ pb)
 {
+    const int NZp = padded_nz(C < 2 ? P.nz + 2 : P.nz + 1);
     const int NZ = C < 2 ? P.nz + 2 : P.nz + 1;
     const int PX = P.nx + kBX, PY = P.ny + kBY;
     const int rows = PX * PY;
@@ -429,12 +433,25 @@ __global__ void __launch_bounds__(256) k_mid_pack(SlcParams P, const double *__r
             if (z < NZ) {
                 va = ra[z];
                 vb = rb[z];
-                if (dm) dm[z] = ca * va + cb * vb;
+                if (dm) dm[z] = fma(2.0, va, -vb);
             }
             da[z] = va;
             db[z] = vb;
         }
     }
+}
+
+struct MidPack {
+    const double *a[3], *b[3];
+    double *mid[3], *pad[6];
+};
+
+__global__ void __launch_bounds__(256) k_mid_pack(const __grid_constant__ SlcParams P,
+                                                  const __grid_constant__ MidPack a)
+{
+    if (blockIdx.y == 0) mid_pack<0>(P, a.a[0], a.b[0], a.mid[0], a.pad[0], a.pad[3]);
+    else if (blockIdx.y == 1) mid_pack<1>(P, a.a[1], a.b[1], a.mid[1], a.pad[1], a.pad[4]);
+    else mid_pack<2>(P, a.a[2], a.b[2], a.mid[2], a.pad[2], a.pad[5]);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -474,10 +491,10 @@ cudaError_t launch_tma_t(const SlcParams &P, const Vel3 &M, Tri fn, Tri fnm1, do
             e = cudaFuncSetAttribute(k_sl_tma_seq<2, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
         const CUtensorMap *tq = (const CUtensorMap *)T.maps;
-        k_sl_tma_seq<0, O><<<gc, kThreads, sm, s>>>(P, M, fn.u, fnm1.u, dt, out.u, ncl, stats, tq[0], tq[3]);
-        k_sl_tma_seq<1, O><<<gc, kThreads, sm, s>>>(P, M, fn.v, fnm1.v, dt, out.v, ncl, stats, tq[1], tq[4]);
+        launch_chained(k_sl_tma_seq<0, O>, gc, kThreads, sm, s, false, P, M, fn.u, fnm1.u, dt, out.u, ncl, stats, tq[0], tq[3]);
+        launch_chained(k_sl_tma_seq<1, O>, gc, kThreads, sm, s, true, P, M, fn.v, fnm1.v, dt, out.v, ncl, stats, tq[1], tq[4]);
         if (P.nz > 1)
-            k_sl_tma_seq<2, O><<<gw, kThreads, sm, s>>>(P, M, fn.w, fnm1.w, dt, out.w, ncl, stats, tq[2], tq[5]);
+            launch_chained(k_sl_tma_seq<2, O>, gw, kThreads, sm, s, true, P, M, fn.w, fnm1.w, dt, out.w, ncl, stats, tq[2], tq[5]);
         count_launches(P.nz > 1 ? 3 : 2);
         return cudaGetLastError();
     } else {  // both boxes at once
@@ -499,15 +516,13 @@ cudaError_t launch_tma_t(const SlcParams &P, const Vel3 &M, Tri fn, Tri fnm1, do
 
 }  // namespace
 
-int tma_padded_nz(int NZ) { return (NZ + 1) & ~1; }
-
 // Boxes must fit inside the padded arrays in every dimension.
 bool tma_supported(const SlcParams &P) { return P.nz + 1 >= kBZ && encode_fn() != nullptr; }
 
 size_t tma_padded_elems(const SlcParams &P, int comp)
 {
     const int NZ = comp < 2 ? P.nz + 2 : P.nz + 1;
-    return (size_t)(P.nx + kBX) * (P.ny + kBY) * tma_padded_nz(NZ);
+    return (size_t)(P.nx + kBX) * (P.ny + kBY) * padded_nz(NZ);
 }
 
 // Tensor maps of the six padded node copies (slot comp + 3 * which).
@@ -520,7 +535,7 @@ cudaError_t tma_encode(const SlcParams &P, TmaSL &T)
     for (int q = 0; q < 6; ++q) {
         const int comp = q % 3;
         const int NZ = comp < 2 ? P.nz + 2 : P.nz + 1;
-        const cuuint64_t nzp = (cuuint64_t)tma_padded_nz(NZ);
+        const cuuint64_t nzp = (cuuint64_t)padded_nz(NZ);
         const cuuint64_t dims[3] = {nzp, (cuuint64_t)(P.ny + kBY), (cuuint64_t)(P.nx + kBX)};
         const cuuint64_t strides[2] = {nzp * 8, nzp * 8 * (cuuint64_t)(P.ny + kBY)};
         const bool o4 = P.order == 4;
@@ -538,20 +553,13 @@ cudaError_t tma_encode(const SlcParams &P, TmaSL &T)
 cudaError_t launch_mid_pack(const SlcParams &P, Tri cur, Tri prev, TriMut mid, const TmaSL &T,
                             cudaStream_t s)
 {
-    for (int c = 0; c < 3; ++c) {
-        const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
-        const int nzp = tma_padded_nz(NZ);
-        const long long rows = (long long)(P.nx + kBX) * (P.ny + kBY);
-        long long blocks = (rows + 7) / 8;  // 8 warps, one padded row each
-        if (blocks > 148 * 16) blocks = 148 * 16;
-        const double *a = c == 0 ? cur.u : (c == 1 ? cur.v : cur.w);
-        const double *b = c == 0 ? prev.u : (c == 1 ? prev.v : prev.w);
-        double *m = c == 0 ? mid.u : (c == 1 ? mid.v : mid.w);
-        if (c == 0) k_mid_pack<0><<<(unsigned)blocks, 256, 0, s>>>(P, a, b, 2.0, -1.0, m, T.pad[c], T.pad[c + 3], nzp);
-        else if (c == 1) k_mid_pack<1><<<(unsigned)blocks, 256, 0, s>>>(P, a, b, 2.0, -1.0, m, T.pad[c], T.pad[c + 3], nzp);
-        else k_mid_pack<2><<<(unsigned)blocks, 256, 0, s>>>(P, a, b, 2.0, -1.0, m, T.pad[c], T.pad[c + 3], nzp);
-    }
-    count_launches(3);
+    const long long rows = (long long)(P.nx + kBX) * (P.ny + kBY);
+    long long blocks = (rows + 7) / 8;  // 8 warps, one padded row each
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    const MidPack a{{cur.u, cur.v, cur.w}, {prev.u, prev.v, prev.w}, {mid.u, mid.v, mid.w},
+                    {T.pad[0], T.pad[1], T.pad[2], T.pad[3], T.pad[4], T.pad[5]}};
+    k_mid_pack<<<dim3((unsigned)blocks, 3), 256, 0, s>>>(P, a);
+    count_launches(1);
     return cudaGetLastError();
 }
 

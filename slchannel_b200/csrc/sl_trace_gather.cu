@@ -13,6 +13,8 @@
 // 4/3 ubar - 1/3 ubarbar + dt_eff (2 R^n - R^{n-1}) with the explicit x,y
 // diffusion R evaluated at the arrival point (operators.py:293-367,
 // solver.py:846-903).
+#include <algorithm>
+
 #include "slc_internal.h"
 
 namespace {
@@ -102,9 +104,11 @@ __global__ void __launch_bounds__(kThreads, O == 4 ? SLC_SL_O4_MIN_BLOCKS : SLC_
     const int k = blockIdx.x * kTileK + (threadIdx.x % kTileK);
     const int j = blockIdx.y * kTileJ + (threadIdx.x / kTileK);
     const int i = blockIdx.z;
+    overlap_begin();
     unsigned ncl = 0;
     sl_point<C, O, MODE, TO, O == 4>(P, M, fn, fnm1, dt, out, i, j, k, ncl);
     add_clamps(nclamp, ncl);
+    overlap_end();
 }
 
 // The slab-streamed forms of k_sl's BDF2 mode (host_step.cu): the same
@@ -180,6 +184,7 @@ __global__ void __launch_bounds__(kThreads) k_advect_multi(const __grid_constant
     const int j = blockIdx.y * kTileJ + (threadIdx.x / kTileK);
     const int i = blockIdx.z;
     const int nzi = (C == 2) ? P.nz - 1 : P.nz;
+    overlap_begin();
     unsigned ncl = 0;
     if (k < nzi && j < P.ny) {
         double xa, ya, za;
@@ -206,6 +211,7 @@ __global__ void __launch_bounds__(kThreads) k_advect_multi(const __grid_constant
         }
     }
     if (nclamp) add_clamps(nclamp, ncl);
+    overlap_end();
 }
 
 template <int C>
@@ -261,6 +267,18 @@ __global__ void k_lincomb(const double *__restrict__ a, const double *__restrict
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
          p += (long long)gridDim.x * blockDim.x)
         out[p] = ca * a[p] + cb * b[p];
+}
+
+__global__ void k_star(Tri a, Tri b, TriMut out, long long n0, long long n1, long long n2)
+{
+    const int c = blockIdx.y;
+    const double *__restrict__ pa = c == 0 ? a.u : (c == 1 ? a.v : a.w);
+    const double *__restrict__ pb = c == 0 ? b.u : (c == 1 ? b.v : b.w);
+    double *__restrict__ o = c == 0 ? out.u : (c == 1 ? out.v : out.w);
+    const long long n = c == 0 ? n0 : (c == 1 ? n1 : n2);
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
+         p += (long long)gridDim.x * blockDim.x)
+        o[p] = fma(2.0, pa[p], -pb[p]);
 }
 
 inline unsigned blocks_for(long long n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
@@ -351,9 +369,9 @@ void launch_sl_tt(const SlcParams &P, const Vel3 &M, Tri fn, Tri fnm1, double dt
 {
     const dim3 gc((P.nz + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
     const dim3 gw((P.nz - 1 + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
-    k_sl<0, O, MODE, TO><<<gc, kThreads, 0, s>>>(P, M, fn.u, fnm1.u, dt, out.u, ncl);
-    k_sl<1, O, MODE, TO><<<gc, kThreads, 0, s>>>(P, M, fn.v, fnm1.v, dt, out.v, ncl);
-    if (P.nz > 1) k_sl<2, O, MODE, TO><<<gw, kThreads, 0, s>>>(P, M, fn.w, fnm1.w, dt, out.w, ncl);
+    launch_chained(k_sl<0, O, MODE, TO>, gc, kThreads, 0, s, false, P, M, fn.u, fnm1.u, dt, out.u, ncl);
+    launch_chained(k_sl<1, O, MODE, TO>, gc, kThreads, 0, s, true, P, M, fn.v, fnm1.v, dt, out.v, ncl);
+    if (P.nz > 1) launch_chained(k_sl<2, O, MODE, TO>, gw, kThreads, 0, s, true, P, M, fn.w, fnm1.w, dt, out.w, ncl);
     count_launches(P.nz > 1 ? 3 : 2);
 }
 
@@ -446,9 +464,9 @@ void launch_multi_t(const SlcParams &P, const MultiIO *io, const Vel3 &M, double
 {
     const dim3 gc((P.nz + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
     const dim3 gw((P.nz - 1 + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
-    k_advect_multi<0, O, TO><<<gc, kThreads, 0, s>>>(P, M, io[0], dt, ncl);
-    k_advect_multi<1, O, TO><<<gc, kThreads, 0, s>>>(P, M, io[1], dt, ncl);
-    if (P.nz > 1) k_advect_multi<2, O, TO><<<gw, kThreads, 0, s>>>(P, M, io[2], dt, ncl);
+    launch_chained(k_advect_multi<0, O, TO>, gc, kThreads, 0, s, false, P, M, io[0], dt, ncl);
+    launch_chained(k_advect_multi<1, O, TO>, gc, kThreads, 0, s, true, P, M, io[1], dt, ncl);
+    if (P.nz > 1) launch_chained(k_advect_multi<2, O, TO>, gw, kThreads, 0, s, true, P, M, io[2], dt, ncl);
     count_launches(P.nz > 1 ? 3 : 2);
 }
 }  // namespace
@@ -524,6 +542,14 @@ cudaError_t launch_face_coord(const SlcParams &P, const double *z, int64_t n, do
 {
     if (n <= 0) return cudaSuccess;
     k_face_coord<<<blocks_for(n), kThreads, 0, s>>>(P, z, n, kf);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_star(Tri cur, Tri prev, TriMut star, const size_t n[3], cudaStream_t s)
+{
+    const unsigned blocks = std::min(blocks_for((long long)std::max(n[0], std::max(n[1], n[2]))), 148u * 16u);
+    k_star<<<dim3(blocks, 3), kThreads, 0, s>>>(cur, prev, star, (long long)n[0], (long long)n[1], (long long)n[2]);
     count_launches(1);
     return cudaGetLastError();
 }

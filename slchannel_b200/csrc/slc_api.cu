@@ -480,9 +480,9 @@ int do_trace_gather_bdf2(slc_grid *g, const double *const cur[3], const double *
         return SLC_OK;
     }
     long t = tim_begin(g, SLC_PHASE_MID, s);
-    for (int c = 0; c < 3; ++c)
-        SLC_CK(launch_lincomb(cur[c], prev[c], 2.0, -1.0, g->mid[c], (int64_t)g->ghost_elems[c], s),
-               "U* = 2V^n - V^{n-1}");
+    SLC_CK(launch_star(Tri{cur[0], cur[1], cur[2]}, Tri{prev[0], prev[1], prev[2]},
+                       TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->ghost_elems, s),
+           "U* = 2V^n - V^{n-1}");
     tim_end(g, t, s);
     unsigned long long *ncl = counter(g, nclamp);
     SLC_CK(cudaMemsetAsync(ncl, 0, sizeof(unsigned long long), s), "memset");
@@ -717,7 +717,9 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     CREATE_CK(dalloc(g, &g->partials, (size_t)kBulkBlocks, "bulk partials"));
     CREATE_CK(dalloc(g, &g->scal, (size_t)8, "scalars"));
     CREATE_CK(dalloc(g, &g->dev_flags, (size_t)4, "device flags"));
-    if (cudaMemset(g->dev_flags, 0, 4 * sizeof(unsigned long long)) != cudaSuccess) {
+    CREATE_CK(dalloc(g, &g->ticket, (size_t)1, "bulk ticket"));
+    if (cudaMemset(g->dev_flags, 0, 4 * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemset(g->ticket, 0, sizeof(unsigned)) != cudaSuccess) {
         slc_grid_destroy(g);
         return fail(nullptr, SLC_E_CUDA, "memset device flags");
     }
@@ -1006,8 +1008,9 @@ int slc_bulk_velocity(slc_grid *g, const double *u, double *out, void *stream)
     if (!u || !out) return fail(g, SLC_E_INVALID, "null pointer");
     DeviceGuard dg(g->device);
     cudaStream_t s = S(stream);
-    SLC_CK(launch_bulk_partials(g->P, (double *)u, g->dzf, nullptr, g->partials, s), "bulk");
-    SLC_CK(launch_bulk_finish(g->P, g->partials, g->Lx, g->Ly, 0.0, 1.0, out, nullptr, s), "bulk");
+    SLC_CK(launch_bulk_sum(g->P, (double *)u, g->dzf, nullptr, g->partials, g->ticket, g->Lx, g->Ly, 0.0, 1.0, out,
+                           nullptr, s),
+           "bulk");
     return SLC_OK;
 }
 
@@ -1061,14 +1064,12 @@ int slc_bulk_shift(slc_grid *g, double *u, double *v, double *w, double U_bulk, 
     DeviceGuard dg(g->device);
     cudaStream_t s = S(stream);
     long t = tim_begin(g, SLC_PHASE_BULK, s);
-    SLC_CK(launch_bulk_partials(g->P, u, g->dzf, nullptr, g->partials, s), "bulk");
-    SLC_CK(launch_bulk_finish(g->P, g->partials, g->Lx, g->Ly, U_bulk, dt, nullptr, g->scal, s),
+    SLC_CK(launch_bulk_sum(g->P, u, g->dzf, nullptr, g->partials, g->ticket, g->Lx, g->Ly, U_bulk, dt, nullptr,
+                           g->scal, s),
            "bulk");
-    SLC_CK(launch_bulk_partials(g->P, u, g->dzf, g->scal, g->partials, s), "bulk shift");
+    SLC_CK(launch_bulk_sum(g->P, u, g->dzf, g->scal, g->partials, g->ticket, g->Lx, g->Ly, 0.0, 1.0, out2, nullptr, s),
+           "bulk shift");
     SLC_CK(launch_apply_bc(g->P, u, v, w, nullptr, s), "boundary conditions");
-    SLC_CK(launch_bulk_finish(g->P, g->partials, g->Lx, g->Ly, 0.0, 1.0, out2, nullptr, s), "bulk");
-    SLC_CK(cudaMemcpyAsync(out2 + 1, g->scal + 1, sizeof(double), cudaMemcpyDeviceToDevice, s),
-           "copy forcing");
     tim_end(g, t, s);
     return SLC_OK;
 }

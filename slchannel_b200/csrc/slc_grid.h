@@ -42,6 +42,7 @@ struct slc_grid {
     double zs_dt = 0.0;
     bool zs_valid = false;
     double *partials = nullptr, *scal = nullptr;
+    unsigned *ticket = nullptr;  // launch_bulk_sum's counter, 0 between launches
     unsigned long long *ncl_scratch = nullptr;
     double *mid[3] = {nullptr, nullptr, nullptr};
     int mixed = 0;          // SLC_PREC_MIXED

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 
 #include "slc_common.cuh"
 
@@ -20,6 +21,41 @@ struct Tri {
 struct TriMut {
     double *u, *v, *w;
 };
+
+// The trace+gather kernels of the three components read the same fields and
+// write different ones.  Launched as a chain of programmatic dependents they
+// overlap: every block lets the next launch begin at once (overlap_begin), so the
+// next component's blocks fill the slots that the last, partly filled wave of
+// this one leaves, and at its end waits for the launches before it
+// (overlap_end), so the last launch's completion is that of all.  A small grid
+// is three part waves side by side instead of one after the other.  Both are
+// no-ops in a kernel launched the ordinary way.
+__device__ __forceinline__ void overlap_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void overlap_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch kernel on s; with overlap, as a programmatic dependent of the launch
+// before it on s (which must be a kernel that calls overlap_begin and
+// overlap_end and writes nothing this one reads).  A stream under capture gets
+// ordinary launches.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool overlap,
+                           A &&...args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (overlap && cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) {
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // ---- sl_trace_gather.cu ----------------------------------------------------
 // mode: 0 = one foot (advect), 1 = BDF1 predictor, 2 = BDF2 predictor.
@@ -43,6 +79,8 @@ cudaError_t launch_interp(const SlcParams &P, int comp, int order, const double 
                           cudaStream_t s);
 cudaError_t launch_face_coord(const SlcParams &P, const double *z, int64_t n, double *kf,
                               cudaStream_t s);
+// U* = 2 V^n - V^{n-1} of all three components (n elements each) in one launch.
+cudaError_t launch_star(Tri cur, Tri prev, TriMut star, const size_t n[3], cudaStream_t s);
 cudaError_t launch_lincomb(const double *a, const double *b, double ca, double cb, double *out,
                            int64_t n, cudaStream_t s);
 
@@ -90,12 +128,24 @@ cudaError_t launch_bulk_partials(const SlcParams &P, double *u, const double *dz
 cudaError_t launch_bulk_finish(const SlcParams &P, const double *partials, double Lx, double Ly,
                                double U_bulk, double dt, double *bulk_out, double *shift_out,
                                cudaStream_t s);
+// The same in one launch (ticket: a zeroed counter, zero again afterwards);
+// with c_dev, bulk_out has a second entry that receives c_dev[1].
+cudaError_t launch_bulk_sum(const SlcParams &P, double *u, const double *dz_f, const double *c_dev,
+                            double *partials, unsigned *ticket, double Lx, double Ly, double U_bulk, double dt,
+                            double *bulk_out, double *shift_out, cudaStream_t s);
 
 // u, v, w interiors -= c grad(p) for a ghost-shaped p (the inc branch).
 cudaError_t launch_grad_sub(const SlcParams &P, const double *p, TriMut f, const double *dz_c, double c,
                             cudaStream_t s);
 
-constexpr int kBulkBlocks = 1184;  // 8 x 148 SMs; fixed, so the sum order is too
+constexpr int kBulkBlocks = 1184;  // 8 x 148 SMs
+// Blocks of the bulk sums: four columns in flight each, at most kBulkBlocks; a
+// function of the grid alone, so the order of the sum is fixed.
+__host__ __device__ inline int bulk_blocks(int nx, int ny)
+{
+    const int need = (nx * ny + 3) / 4;
+    return need < kBulkBlocks ? need : kBulkBlocks;
+}
 
 // Message of a failed handle-free call, for slc_last_error(NULL); returns code.
 int slc_report_error(int code, const char *msg);
@@ -190,7 +240,6 @@ struct TmaSL {
     double *pad[6];
     alignas(64) unsigned char maps[6 * 128];
 };
-int tma_padded_nz(int NZ);
 size_t tma_padded_elems(const SlcParams &P, int comp);
 bool tma_supported(const SlcParams &P);
 cudaError_t tma_encode(const SlcParams &P, TmaSL &T);
