@@ -62,6 +62,12 @@ struct slc_ensemble {
 
 // An order-6 instance whose staged trace+gather has at least this many
 // blocks per component (a few waves of the GPU) runs it as its own launches.
+// It gathers from boxes while the mean flow moves less than this many cells per
+// step, through L1 alone above: the boxes leave three cells of spread in y and z,
+// which the fluctuations of a flow that moves further exceed in many blocks
+// (128x64x128 at 1.8 cells: a third of the far boxes; staged 3.5 ms, L1 2.6 ms
+// for the three such instances of the 12-channel benchmark ensemble).
+constexpr double kEnsBoxCells = 1.5;
 #ifndef SLC_ENS_STAGED_MIN_BLOCKS
 #define SLC_ENS_STAGED_MIN_BLOCKS 2048
 #endif
@@ -133,6 +139,13 @@ void free_groups(slc_ensemble *e)
             cufftDestroy(gr.inv);
             gr.plans = false;
         }
+}
+
+// Blocks per component of an instance's staged trace+gather.
+long long staged_blocks(const SlcParams &P, bool mixed)
+{
+    if (mixed) return (long long)((P.nz + 31) / 32) * ((P.ny + 3) / 4) * ((P.nx + 1) / 2);
+    return (long long)((P.nx + 31) / 32) * ((P.ny + 1) / 2) * ((P.nz + 3) / 4);
 }
 
 // Work items of every multi-instance kernel, in one array.
@@ -301,8 +314,8 @@ int enqueue_step(slc_ensemble *e, int ph, cudaStream_t s)
         } else {
             ENS_CK(launch_mid_pack(g->P, a, b, TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->tma, s),
                    "U* and padded node copies");
-            ENS_CK(launch_sl_tma(g->P, a, b, Tri{g->mid[0], g->mid[1], g->mid[2]}, H.dt, o, H.ncl, g->dev_flags,
-                                 g->tma, s),
+            ENS_CK(launch_sl_tma(g->P, Tri{g->mid[0], g->mid[1], g->mid[2]}, H.dt, o, H.ncl, g->dev_flags,
+                                 g->tma, H.dt * H.U_bulk * g->P.inv_dx < kEnsBoxCells, s),
                    "trace+gather BDF2 (TMA-staged)");
         }
     }
@@ -533,7 +546,7 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
     if (e->order == 6)
         for (int i = 0; i < n; ++i) {
             const SlcParams &P = e->grids[i]->P;
-            const long long blocks = (long long)((P.nz + 31) / 32) * ((P.ny + 3) / 4) * ((P.nx + 1) / 2);
+            const long long blocks = staged_blocks(P, e->mixed);
             if (blocks < SLC_ENS_STAGED_MIN_BLOCKS) continue;
             bool ready = false;
             int rs = slc_grid_ensure_staged(e->grids[i], &ready);

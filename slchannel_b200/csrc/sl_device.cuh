@@ -6,6 +6,9 @@
 struct Vel3 {
     NodeView<double> u, v, w;
 };
+struct Vel3X {  // x fastest
+    NodeViewX u, v, w;
+};
 
 __device__ __forceinline__ void add_clamps(unsigned long long *counter, unsigned cnt)
 {
@@ -15,7 +18,8 @@ __device__ __forceinline__ void add_clamps(unsigned long long *counter, unsigned
 
 // Trajectory velocity at one point (semilag.py:512-528, traj_order = 2):
 // z clamped to [z_lo, z_hi], one face-locate shared by the three samples.
-__device__ __forceinline__ void sample3(const SlcParams &P, const Vel3 &M, double x, double y,
+template <class V3>
+__device__ __forceinline__ void sample3(const SlcParams &P, const V3 &M, double x, double y,
                                         double z, double &us, double &vs, double &ws)
 {
     const double zc = clampz(P, z);
@@ -30,18 +34,26 @@ __device__ __forceinline__ void sample3(const SlcParams &P, const Vel3 &M, doubl
 // semilag.py:206-209, 512-528): the order-4 tensor-product stencils of the
 // field gather on the three trajectory components.  Kept out of line so the
 // trilinear path's register allocation does not carry it.
-__device__ __noinline__ void sample3_o4(const SlcParams &P, const Vel3 &M, double x, double y,
+template <typename T>
+__device__ __forceinline__ int x_step(const NodeView<T> &V)
+{
+    return V.sx;
+}
+__device__ __forceinline__ int x_step(const NodeViewX &) { return 1; }
+
+template <class V3>
+__device__ __noinline__ void sample3_o4(const SlcParams &P, const V3 &M, double x, double y,
                                         double z, double &us, double &vs, double &ws)
 {
     const double zc = clampz(P, z);
     const int c = half_cell(P, zc);
     Stencil<4, double> st;
-    build_stencil<0, 4, double>(P, M.u.sx, M.u.sy, x, y, zc, c, st);
-    us = gather_sum<4, double, double>(M.u.p, st);
-    build_stencil<1, 4, double>(P, M.v.sx, M.v.sy, x, y, zc, c, st);
-    vs = gather_sum<4, double, double>(M.v.p, st);
-    build_stencil<2, 4, double>(P, M.w.sx, M.w.sy, x, y, zc, c, st);
-    ws = gather_sum<4, double, double>(M.w.p, st);
+    build_stencil<0, 4, double>(P, x_step(M.u), M.u.sy, x, y, zc, c, st);
+    us = gather_sum<4, double, double>(M.u.p, st, z_step(M.u));
+    build_stencil<1, 4, double>(P, x_step(M.v), M.v.sy, x, y, zc, c, st);
+    vs = gather_sum<4, double, double>(M.v.p, st, z_step(M.v));
+    build_stencil<2, 4, double>(P, x_step(M.w), M.w.sy, x, y, zc, c, st);
+    ws = gather_sum<4, double, double>(M.w.p, st, z_step(M.w));
 }
 
 // Trajectory sampling order as a template argument: 2 or 4 fixed at compile
@@ -54,8 +66,8 @@ __device__ __forceinline__ bool traj4(const SlcParams &P)
 
 // First fixed-point sample at the arrival point (i, j, k) of component C:
 // exact node values for trilinear sampling, the stencils for tricubic.
-template <int C, int TO = 0>
-__device__ __forceinline__ void first_sample(const SlcParams &P, const Vel3 &M, int i, int j, int k,
+template <int C, int TO = 0, class V3>
+__device__ __forceinline__ void first_sample(const SlcParams &P, const V3 &M, int i, int j, int k,
                                              double xa, double ya, double za, double &us0,
                                              double &vs0, double &ws0)
 {
@@ -67,8 +79,8 @@ __device__ __forceinline__ void first_sample(const SlcParams &P, const Vel3 &M, 
 // (us0, vs0, ws0) taken at the arrival point; returns the unclamped foot.
 // NI: the number of iterations at compile time (no loop, so that the samples
 // of several feet can be in flight together), 0 to read P.n_iters.
-template <int TO = 0, int NI = 0>
-__device__ __forceinline__ void trace_foot(const SlcParams &P, const Vel3 &M, double xa, double ya,
+template <int TO = 0, int NI = 0, class V3>
+__device__ __forceinline__ void trace_foot(const SlcParams &P, const V3 &M, double xa, double ya,
                                            double za, double half_dt, double us0, double vs0,
                                            double ws0, double &xd, double &yd, double &zd)
 {
@@ -136,3 +148,25 @@ __device__ __forceinline__ double bdf2_combine(double ubar, double ubb, double d
     return fma((2.0 / 3.0) * dt, Rh, dot2(ubar, 4.0 / 3.0, ubb, -1.0 / 3.0));
 }
 
+// The same from a node view with x fastest (periodic wrap by index).
+template <int C>
+__device__ __forceinline__ double xy_diffusion(const SlcParams &P, const NodeViewX &F, int i, int j, int k)
+{
+    // arrival point (i, j, k) is node (i + 1, j) of u, (i, j + 1) of v, (i, j)
+    // of w, at level k + 1
+    const int I = C == 0 ? (i + 1 == P.nx ? 0 : i + 1) : i, J = C == 1 ? (j + 1 == P.ny ? 0 : j + 1) : j;
+    const int Im = I == 0 ? P.nx - 1 : I - 1, Ip = I + 1 == P.nx ? 0 : I + 1;
+    const int Jm = J == 0 ? P.ny - 1 : J - 1, Jp = J + 1 == P.ny ? 0 : J + 1;
+    const double fc = __ldg(node_at(F, I, J, k + 1));
+    const double d2x = fma(-2.0, fc, __ldg(node_at(F, Ip, J, k + 1))) + __ldg(node_at(F, Im, J, k + 1));
+    const double d2y = fma(-2.0, fc, __ldg(node_at(F, I, Jp, k + 1))) + __ldg(node_at(F, I, Jm, k + 1));
+    return __dmul_rn(P.nu, dot2(d2x, P.inv_dx2, d2y, P.inv_dy2));
+}
+
+template <int C>
+__device__ __forceinline__ double xy_diffusion_bdf2(const SlcParams &P, const NodeViewX &fn, const NodeViewX &fnm1,
+                                                    int i, int j, int k)
+{
+    const double Rn = xy_diffusion<C>(P, fn, i, j, k);
+    return P.xy_lagged ? Rn : fma(2.0, Rn, -xy_diffusion<C>(P, fnm1, i, j, k));
+}

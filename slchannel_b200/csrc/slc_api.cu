@@ -341,12 +341,6 @@ enum GatherMode { kGatherDefault, kGatherL1, kGatherStaged };
 #ifndef SLC_MIXED_STAGED_DEFAULT  // the mixed step gathers from TMA-staged boxes
 #define SLC_MIXED_STAGED_DEFAULT 1
 #endif
-#ifndef SLC_FP64_STAGED_DEFAULT  // so does the FP64 step at order 6
-#define SLC_FP64_STAGED_DEFAULT 1
-#endif
-#ifndef SLC_FP64_O4_STAGED_DEFAULT  // and at order 4
-#define SLC_FP64_O4_STAGED_DEFAULT 0
-#endif
 // The step keeps gathering from staged boxes while at least this fraction of
 // the blocks staged both feet, and otherwise gathers through L1 (whose
 // kernel holds more registers per thread, so it is the faster when many
@@ -454,15 +448,16 @@ int do_trace_gather_bdf2(slc_grid *g, const double *const cur[3], const double *
         tim_end(g, t, s);
         return SLC_OK;
     }
-    // the FP64 staged kernel holds three blocks per SM; at order 4 the L1
-    // kernel runs four and stays the faster
-    bool staged = mode == kGatherStaged ||
-                  (mode == kGatherDefault && (g->P.order == 6 ? SLC_FP64_STAGED_DEFAULT : SLC_FP64_O4_STAGED_DEFAULT));
+    // By default an order-6 step reads the fields through copies with x fastest,
+    // from boxes while the feet fit them (choose_staged), else through L1 alone;
+    // order 4 keeps k_sl (64 loads per foot leave too little to save).
+    const bool copies = mode == kGatherStaged || (mode == kGatherDefault && g->P.order == 6);
     int rc = ensure_mid(g);
-    if (!rc && staged) rc = ensure_tma(g);
+    if (!rc && copies) rc = ensure_tma(g);
     if (rc) return rc;
-    if (staged && mode == kGatherDefault && g->tma_state == 1) staged = choose_staged(g, s);
-    if (staged && g->tma_state == 1) {
+    const bool by_x = copies && g->tma_state == 1;
+    const bool staged = by_x && (mode == kGatherStaged || choose_staged(g, s));
+    if (by_x) {
         long t = tim_begin(g, SLC_PHASE_MID, s);
         SLC_CK(launch_mid_pack(g->P, Tri{cur[0], cur[1], cur[2]}, Tri{prev[0], prev[1], prev[2]},
                                TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->tma, s),
@@ -471,12 +466,11 @@ int do_trace_gather_bdf2(slc_grid *g, const double *const cur[3], const double *
         unsigned long long *ncl = counter(g, nclamp);
         SLC_CK(cudaMemsetAsync(ncl, 0, sizeof(unsigned long long), s), "memset");
         t = tim_begin(g, SLC_PHASE_SL, s);
-        SLC_CK(launch_sl_tma(g->P, Tri{cur[0], cur[1], cur[2]}, Tri{prev[0], prev[1], prev[2]},
-                             Tri{g->mid[0], g->mid[1], g->mid[2]}, dt, TriMut{out[0], out[1], out[2]},
-                             ncl, g->dev_flags, g->tma, s),
-               "trace+gather BDF2 (TMA-staged)");
+        SLC_CK(launch_sl_tma(g->P, Tri{g->mid[0], g->mid[1], g->mid[2]}, dt, TriMut{out[0], out[1], out[2]},
+                             ncl, g->dev_flags, g->tma, staged, s),
+               "trace+gather BDF2 (x along the lanes)");
         tim_end(g, t, s);
-        if (mode == kGatherDefault) note_staged(g, s);
+        if (staged && mode == kGatherDefault) note_staged(g, s);
         return SLC_OK;
     }
     long t = tim_begin(g, SLC_PHASE_MID, s);

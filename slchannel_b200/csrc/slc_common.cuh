@@ -54,6 +54,29 @@ struct NodeView {
     int sx, sy;
 };
 
+// The same with x fastest: element = p[i + j*sy + k*sz].
+struct NodeViewX {
+    const double *p;
+    int sy, sz;
+};
+
+// Address of a node and the distance to its upper z neighbour, in either view.
+template <typename T>
+__device__ __forceinline__ const T *node_at(const NodeView<T> &V, int i, int j, int k)
+{
+    return V.p + i * V.sx + j * V.sy + k;
+}
+template <typename T>
+__device__ __forceinline__ int z_step(const NodeView<T> &)
+{
+    return 1;
+}
+__device__ __forceinline__ const double *node_at(const NodeViewX &V, int i, int j, int k)
+{
+    return V.p + i + j * V.sy + k * V.sz;
+}
+__device__ __forceinline__ int z_step(const NodeViewX &V) { return V.sz; }
+
 // Component node grids (semilag.py:258-286): u and v on cell centres incl.
 // the two ghost centres (NZ = nz+2), w on faces incl. walls (NZ = nz+1).
 // Node coordinate s_x = x/dx + shift_x.
@@ -290,8 +313,9 @@ __device__ __forceinline__ void build_stencil(const SlcParams &P, int sx, int sy
 // multiply-adds), the z weights come last (the reference sums the O^3 products
 // in one sequence, semilag.py:44-59; the grouping here differs only by
 // rounding).
+// zs: distance of z neighbours (st's offsets hold those of x and y).
 template <int O, typename T, typename A>
-__device__ __forceinline__ A gather_sum(const T *__restrict__ F, const Stencil<O, T> &st)
+__device__ __forceinline__ A gather_sum(const T *__restrict__ F, const Stencil<O, T> &st, int zs = 1)
 {
     A acc[O];
 #pragma unroll
@@ -300,10 +324,10 @@ __device__ __forceinline__ A gather_sum(const T *__restrict__ F, const Stencil<O
     for (int i = 0; i < O; ++i) {
 #pragma unroll
         for (int j = 0; j < O; ++j) {
-            const T *row = F + st.xoff[i] + st.yoff[j] + st.k0;
+            const T *row = F + st.xoff[i] + st.yoff[j] + st.k0 * zs;
             const A w = (A)st.wx[i] * (A)st.wy[j];
 #pragma unroll
-            for (int k = 0; k < O; ++k) acc[k] = fma(w, (A)__ldg(row + k), acc[k]);
+            for (int k = 0; k < O; ++k) acc[k] = fma(w, (A)__ldg(row + k * zs), acc[k]);
         }
     }
     A r = (A)0;
@@ -314,18 +338,17 @@ __device__ __forceinline__ A gather_sum(const T *__restrict__ F, const Stencil<O
 
 // One trilinear sample of node view V from precomputed corner indices and
 // weights (x: i0, i1, tx; y: j0, j1, ty; z: k0, wz0, wz1).
-template <typename T>
-__device__ __forceinline__ double tri_sample(NodeView<T> V, int i0, int i1, double tx, int j0, int j1,
+template <class View>
+__device__ __forceinline__ double tri_sample(const View &V, int i0, int i1, double tx, int j0, int j1,
                                              double ty, int k0, double wz0, double wz1)
 {
-    const T *p00 = V.p + i0 * V.sx + j0 * V.sy + k0;
-    const T *p01 = V.p + i0 * V.sx + j1 * V.sy + k0;
-    const T *p10 = V.p + i1 * V.sx + j0 * V.sy + k0;
-    const T *p11 = V.p + i1 * V.sx + j1 * V.sy + k0;
-    const double a00 = dot2(wz0, (double)__ldg(p00), wz1, (double)__ldg(p00 + 1));
-    const double a01 = dot2(wz0, (double)__ldg(p01), wz1, (double)__ldg(p01 + 1));
-    const double a10 = dot2(wz0, (double)__ldg(p10), wz1, (double)__ldg(p10 + 1));
-    const double a11 = dot2(wz0, (double)__ldg(p11), wz1, (double)__ldg(p11 + 1));
+    const auto *p00 = node_at(V, i0, j0, k0), *p01 = node_at(V, i0, j1, k0);
+    const auto *p10 = node_at(V, i1, j0, k0), *p11 = node_at(V, i1, j1, k0);
+    const int up = z_step(V);
+    const double a00 = dot2(wz0, (double)__ldg(p00), wz1, (double)__ldg(p00 + up));
+    const double a01 = dot2(wz0, (double)__ldg(p01), wz1, (double)__ldg(p01 + up));
+    const double a10 = dot2(wz0, (double)__ldg(p10), wz1, (double)__ldg(p10 + up));
+    const double a11 = dot2(wz0, (double)__ldg(p11), wz1, (double)__ldg(p11 + up));
     const double wx0 = 1.0 - tx, wy0 = 1.0 - ty;
     return dot2(wx0, dot2(wy0, a00, ty, a01), tx, dot2(wy0, a10, ty, a11));
 }
@@ -377,9 +400,10 @@ __device__ __forceinline__ void tri_shared(const SlcParams &P, double x, double 
 
 // Node value accessor for the arrival-point sample below (FP64 node views).
 struct NodeValF64 {
-    __device__ __forceinline__ double operator()(NodeView<double> V, int I, int J, int K) const
+    template <class View>
+    __device__ __forceinline__ double operator()(const View &V, int I, int J, int K) const
     {
-        return __ldg(V.p + I * V.sx + J * V.sy + K);
+        return __ldg(node_at(V, I, J, K));
     }
 };
 

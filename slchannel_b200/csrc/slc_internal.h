@@ -243,15 +243,15 @@ struct TmaSL {
 size_t tma_padded_elems(const SlcParams &P, int comp);
 bool tma_supported(const SlcParams &P);
 cudaError_t tma_encode(const SlcParams &P, TmaSL &T);
-// U* (node entries of the ghost-shaped mid arrays) and the padded copies.
+// U* (nodes with x fastest, in the mid arrays) and the padded copies.
 cudaError_t launch_mid_pack(const SlcParams &P, Tri cur, Tri prev, TriMut mid, const TmaSL &T,
                             cudaStream_t s);
 // stats (device, accumulated): [0] staged boxes that did not arrive within
 // the poll limit (that block then gathers through L1; results stay exact),
-// [1] blocks, [2] near-foot boxes staged, [3] far-foot boxes staged.
-cudaError_t launch_sl_tma(const SlcParams &P, Tri fn, Tri fnm1, Tri mid, double dt, TriMut out,
-                          unsigned long long *nclamp, unsigned long long *stats, const TmaSL &T,
-                          cudaStream_t s);
+// [1] blocks, [2] near-foot boxes staged, [3] far-foot boxes staged.  Without
+// staged: through L1 alone, from the same copies.
+cudaError_t launch_sl_tma(const SlcParams &P, Tri mid, double dt, TriMut out, unsigned long long *nclamp,
+                          unsigned long long *stats, const TmaSL &T, bool staged, cudaStream_t s);
 
 // One 3-D tiled tensor map (128 bytes at map128; z innermost, zero fill):
 // FP32 or FP64 elements, dims (z, y, x), y and x strides in bytes, box
