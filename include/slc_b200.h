@@ -189,10 +189,9 @@ SLC_API int slc_host_step_stats(slc_grid *g, int64_t *out4);
  * in shared memory by the Tensor Memory Accelerator (3-D cp.async.bulk.tensor
  * loads of halo-padded node copies; otherwise identical to
  * slc_trace_gather_bdf2).  Results are bit-identical to
- * slc_trace_gather_bdf2's.  FP64 handles (nz >= 47): the padded copies are
- * written with U*; not the FP64 step's default, since at the 256^3
- * benchmark that extra pass takes back the kernel's gain, while where the
- * feet spread (trajectory CFL 3) this call is the faster of the two.  Mixed
+ * slc_trace_gather_bdf2's.  FP64 handles (nz >= 47 or nx >= 32): U* and the
+ * padded copies are written with x fastest, and x runs along the lanes;
+ * slc_step_bdf2 at order 6 gathers this way while the feet fit.  Mixed
  * handles (nz >= 62): FP32 fluctuation boxes, the padded copies written by
  * the mixed pack itself; slc_step_bdf2 on a mixed handle gathers this way.
  * slc_gather_stats reports how many boxes were staged.  Synchronous: it

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) k_slab_prep(SlcParams P, PrepJob job, Sla
             } else {
                 a = cur[base + K];
             }
-            const double m = 2.0 * a + (-1.0) * prev[base + K];  // k_lincomb's U*, exactly
+            const double m = 2.0 * a + (-1.0) * prev[base + K];  // k_star's U*, exactly
             mid[base + K] = m;
             if (c == 0) um = max(um, (unsigned long long)__double_as_longlong(fabs(m)));
         }

@@ -33,6 +33,10 @@ constexpr int kTileK = SLC_SLM_TILE_K, kTileJ = kThreads / kTileK;
 #endif
 constexpr int kMeanBlocks = 148;  // column groups of the plane-mean partial sums
 
+// threads per block of the plane means' finish: one level each, so 256 levels of
+// nine fields reach 72 SMs, not 9 (256^3: 35 -> 17 us)
+constexpr int kFinishT = 32;
+
 struct Vel3M {
     MixedView u, v, w;
 };
@@ -722,13 +726,13 @@ struct MeanPtrs {
 
 __device__ __forceinline__ void plane_finish(const SlcParams &P, int nf, const double *partials,
                                              int ldp, int G, double *mean, float *mean32,
-                                             int derived_star, int f)
+                                             int derived_star, int f, int k0, int kstep)
 {
     const int NZ = (f % 3) == 2 ? P.nz + 1 : P.nz + 2;
     const double inv = 1.0 / ((double)P.nx * (double)P.ny);
-    // sums over the G column groups in group order, eight groups' loads in flight
+    // sums over the G column groups in group order, kU groups' loads in flight
     auto group_sum = [&](int fs, int k) {
-        constexpr int kU = 8;
+        constexpr int kU = 16;
         const double *p = partials + (size_t)fs * G * ldp + k;
         double s = 0.0;
         for (int b0 = 0; b0 < G; b0 += kU) {
@@ -741,7 +745,7 @@ __device__ __forceinline__ void plane_finish(const SlcParams &P, int nf, const d
         }
         return s;
     };
-    for (int k = threadIdx.x; k < NZ; k += blockDim.x) {
+    for (int k = k0 + threadIdx.x; k < NZ; k += kstep) {
         double m;
         if (f >= 6 && derived_star) {
             const double sa = group_sum(f - 6, k), sb = group_sum(f - 3, k);
@@ -759,7 +763,7 @@ __global__ void k_plane_finish(SlcParams P, int nf, const double *partials, int 
                                const __grid_constant__ MeanPtrs out, int derived_star)
 {
     plane_finish(P, nf, partials, ldp, G, out.m[blockIdx.x], out.m32[blockIdx.x], derived_star,
-                 blockIdx.x);
+                 blockIdx.x, blockIdx.y * blockDim.x, gridDim.y * blockDim.x);
 }
 
 // FP32 fluctuation node buffers: field slot q = comp (0..2) + 3 * which
@@ -882,13 +886,13 @@ __global__ void __launch_bounds__(256) k_plane_partials_ens(const EnsInst *__res
     plane_partial(I.P, src, f % 3, I.mws.partials, I.P.nz + 2, f, it.a, kMeanBlocks);
 }
 
-// block (inst * 9 + f)
+// block (inst * 9 + f, slice of the levels)
 __global__ void k_plane_finish_ens(const EnsInst *__restrict__ ins)
 {
     const EnsInst &I = ins[blockIdx.x / 9];
     const int f = blockIdx.x % 9;
     plane_finish(I.P, 6, I.mws.partials, I.P.nz + 2, kMeanBlocks, I.mws.mean[f], I.mws.mean32[f], 1,
-                 f);
+                 f, blockIdx.y * blockDim.x, gridDim.y * blockDim.x);
 }
 
 // items (inst, bx, by, bz) as k_pack_mixed's grid
@@ -1019,7 +1023,7 @@ cudaError_t launch_mixed_prepare(const SlcParams &P, Tri A, Tri B, Tri M, const 
         mp.m[f] = ws.mean[f];
         mp.m32[f] = ws.mean32[f];
     }
-    k_plane_finish<<<9, 256, 0, s>>>(P, nf, ws.partials, ldp, kMeanBlocks, mp, explicit_m ? 0 : 1);
+    k_plane_finish<<<dim3(9, (P.nz + 2 + kFinishT - 1) / kFinishT), kFinishT, 0, s>>>(P, nf, ws.partials, ldp, kMeanBlocks, mp, explicit_m ? 0 : 1);
     PackArgs a{};
     for (int c = 0; c < 3; ++c) {
         a.A[c] = src[c];
@@ -1168,7 +1172,7 @@ cudaError_t launch_mixed_prepare_ens(const EnsInst *ins, int ninst, const EnsIte
     // no items: every instance packs its own buffers (the staged gather)
     if (ninst <= 0 || n_pp <= 0 || n_pack <= 0) return cudaSuccess;
     k_plane_partials_ens<<<n_pp, 256, 0, s>>>(ins, pp_items, ph);
-    k_plane_finish_ens<<<9 * ninst, 256, 0, s>>>(ins);
+    k_plane_finish_ens<<<dim3(9 * ninst, 4), kFinishT, 0, s>>>(ins);
     k_pack_mixed_ens<<<n_pack, pack_threads, 0, s>>>(ins, pack_items, ph);
     count_launches(3);
     return cudaGetLastError();

@@ -185,6 +185,16 @@ int do_project(slc_grid *g, double *u, double *v, double *w, double *p, double d
 
 int ensure_mid(slc_grid *g)
 {
+    if (!g->mid[0] && !g->mid[1] && !g->mid[2]) {  // one allocation: each costs a new handle's first call
+        double *p = nullptr;
+        const size_t n = g->ghost_elems[0] + g->ghost_elems[1] + g->ghost_elems[2];
+        int rc = dalloc(g, &p, n, "U* workspace");
+        if (rc) return rc;
+        SLC_CK(cudaMemset(p, 0, n * sizeof(double)), "memset");
+        g->mid[0] = p;
+        g->mid[1] = p + g->ghost_elems[0];
+        g->mid[2] = g->mid[1] + g->ghost_elems[1];
+    }
     for (int c = 0; c < 3; ++c)
         if (!g->mid[c]) {
             int rc = dalloc(g, &g->mid[c], g->ghost_elems[c], "U* workspace");
@@ -204,10 +214,12 @@ int ensure_tma(slc_grid *g)
         g->tma_state = -1;
         return SLC_OK;
     }
-    for (int q = 0; q < 6; ++q) {
-        int rc = dalloc(g, &g->tma.pad[q], tma_padded_elems(g->P, q % 3), "padded node copy");
-        if (rc) return rc;
-    }
+    size_t off[7] = {0};  // one allocation, each copy from a 128-byte boundary (the tensor maps' bases)
+    for (int q = 0; q < 6; ++q) off[q + 1] = off[q] + ((tma_padded_elems(g->P, q % 3) + 15) & ~(size_t)15);
+    double *p = nullptr;
+    int rc = dalloc(g, &p, off[6], "padded node copies");
+    if (rc) return rc;
+    for (int q = 0; q < 6; ++q) g->tma.pad[q] = p + off[q];
     SLC_CK(tma_encode(g->P, g->tma), "tensor map encode");
     g->tma_state = 1;
     return SLC_OK;
@@ -227,12 +239,13 @@ int ensure_mixed_tma(slc_grid *g)
         g->tmx_state = -1;
         return SLC_OK;
     }
-    for (int q = 0; q < 6; ++q) {
-        const size_t n = mixed_tma_elems(g->P, g->mws, q % 3);
-        rc = dalloc(g, &g->tmx.pad[q], n, "padded FP32 copy");
-        if (rc) return rc;
-        SLC_CK(cudaMemset(g->tmx.pad[q], 0, n * sizeof(float)), "memset");
-    }
+    size_t off[7] = {0};  // one allocation, each copy from a 128-byte boundary (the tensor maps' bases)
+    for (int q = 0; q < 6; ++q) off[q + 1] = off[q] + ((mixed_tma_elems(g->P, g->mws, q % 3) + 31) & ~(size_t)31);
+    float *p = nullptr;
+    rc = dalloc(g, &p, off[6], "padded FP32 copies");
+    if (rc) return rc;
+    SLC_CK(cudaMemset(p, 0, off[6] * sizeof(float)), "memset");
+    for (int q = 0; q < 6; ++q) g->tmx.pad[q] = p + off[q];
     if (mixed_tma_encode(g->P, g->mws, g->tmx) != cudaSuccess) {
         g->tmx_state = -1;
         return SLC_OK;
@@ -247,16 +260,21 @@ int ensure_mixed(slc_grid *g)
     const SlcParams &P = g->P;
     g->mws.nzp[0] = g->mws.nzp[1] = mixed_nzp(P.nz + 2);
     g->mws.nzp[2] = mixed_nzp(P.nz + 1);
+    // one allocation for the node buffers and one for the profiles
+    size_t off[10] = {0};
+    for (int q = 0; q < 9; ++q) off[q + 1] = off[q] + (((size_t)P.nx * P.ny * g->mws.nzp[q % 3] + 31) & ~(size_t)31);
+    const size_t levels = ((size_t)P.nz + 2 + 3) & ~(size_t)3;
+    float *nodes = nullptr;
+    double *means = nullptr;
+    int rc = dalloc(g, &nodes, off[9], "mixed FP32 node buffers");
+    if (!rc) rc = dalloc(g, &means, 9 * levels + 9 * levels / 2, "mixed plane means");
+    if (rc) return rc;
     for (int q = 0; q < 9; ++q) {
-        const size_t n = (size_t)P.nx * P.ny * g->mws.nzp[q % 3];
-        int rc = dalloc(g, &g->mws.f32[q], n, "mixed FP32 node buffer");
-        if (rc) return rc;
-        rc = dalloc(g, &g->mws.mean[q], (size_t)P.nz + 2, "mixed plane mean");
-        if (rc) return rc;
-        rc = dalloc(g, &g->mws.mean32[q], (size_t)P.nz + 2, "mixed plane mean fp32");
-        if (rc) return rc;
+        g->mws.f32[q] = nodes + off[q];
+        g->mws.mean[q] = means + q * levels;
+        g->mws.mean32[q] = (float *)(means + 9 * levels) + q * levels;
     }
-    int rc = dalloc(g, &g->mws.partials, mixed_partials_doubles(P), "mixed mean partials");
+    rc = dalloc(g, &g->mws.partials, mixed_partials_doubles(P), "mixed mean partials");
     if (rc) return rc;
     g->mixed_ready = true;
     return SLC_OK;
@@ -625,21 +643,26 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
         std::vector<double> edges;
         std::vector<unsigned short> bins;
         half_cell_bins(P, zc, edges, bins);
+        // one allocation: {node, 1 / interval} of the centres, then of the faces,
+        // the half cells' edges, the bins
+        std::vector<double2> lin = linear_table(zc), lf = linear_table(zf);
+        const size_t nc = lin.size();
+        lin.insert(lin.end(), lf.begin(), lf.end());
+        const size_t ne = (edges.size() + 1) / 2, nb = (bins.size() + 7) / 8;
+        std::vector<double2> all = lin;
+        all.resize(lin.size() + ne + nb);
+        std::memcpy(all.data() + lin.size(), edges.data(), edges.size() * sizeof(double));
+        if (!bins.empty()) std::memcpy(all.data() + lin.size() + ne, bins.data(), bins.size() * sizeof(bins[0]));
+        double2 *d = nullptr;
+        CREATE_CK(upload(g, &d, all, "cell lookup tables"));
+        P.lin_c = d;
+        P.lin_f = d + nc;
         if (!bins.empty()) {
-            double *half = nullptr;
-            unsigned short *bin = nullptr;
-            CREATE_CK(upload(g, &half, edges, "half-cell edges"));
-            CREATE_CK(upload(g, &bin, bins, "half-cell bins"));
-            P.zhalf = half;
-            P.zbin = bin;
+            P.zhalf = (const double *)(d + lin.size());
+            P.zbin = (const unsigned short *)(d + lin.size() + ne);
             P.zbins = (int)bins.size();
             P.zbin_scale = P.zbins / P.Lz;
         }
-        double2 *lin = nullptr;
-        CREATE_CK(upload(g, &lin, linear_table(zc), "centre intervals"));
-        P.lin_c = lin;
-        CREATE_CK(upload(g, &lin, linear_table(zf), "face intervals"));
-        P.lin_f = lin;
     }
     for (int o = 2; o <= SLC_MAX_ORDER; o += 2) {
         if (nz + 2 - o + 1 <= 0) continue;
@@ -696,8 +719,8 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     const size_t nreal = (size_t)nz * nx * ny, ncplx = (size_t)nz * nx * nky;
     CREATE_CK(dalloc(g, &g->rhs, nreal, "Poisson rhs"));
     CREATE_CK(dalloc(g, &g->hat, 2 * ncplx, "Poisson spectrum"));
-    CREATE_CK(dalloc(g, &g->th_id, ncplx, "Poisson elimination factors"));
-    CREATE_CK(dalloc(g, &g->th_g, ncplx, "Poisson elimination factors"));
+    CREATE_CK(dalloc(g, &g->th_id, 2 * ncplx, "Poisson elimination factors"));
+    g->th_g = g->th_id + ncplx;
     {
         // creation is synchronous: later work may come on any stream
         cudaError_t e = launch_thomas_factors(P, g->th_id, g->th_g, g->kx2, g->ky2, g->cl, g->cr, false, 0);
@@ -711,9 +734,9 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     CREATE_CK(dalloc(g, &g->partials, (size_t)kBulkBlocks, "bulk partials"));
     CREATE_CK(dalloc(g, &g->scal, (size_t)8, "scalars"));
     CREATE_CK(dalloc(g, &g->dev_flags, (size_t)4, "device flags"));
-    CREATE_CK(dalloc(g, &g->ticket, (size_t)1, "bulk ticket"));
+    g->ticket = (unsigned *)(g->scal + 7);  // scal[0..1]: shift, forcing
     if (cudaMemset(g->dev_flags, 0, 4 * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemset(g->ticket, 0, sizeof(unsigned)) != cudaSuccess) {
+        cudaMemset(g->scal, 0, 8 * sizeof(double)) != cudaSuccess) {
         slc_grid_destroy(g);
         return fail(nullptr, SLC_E_CUDA, "memset device flags");
     }

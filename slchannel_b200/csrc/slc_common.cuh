@@ -193,7 +193,8 @@ __device__ __forceinline__ double face_coord(const SlcParams &P, double z)
 // bins are lower than the lowest half cell, so a bin holds at most one edge:
 // one lookup and one comparison give the same cell (a z within rounding of a
 // face may land on either side of it, where the interpolants of both cells
-// agree).
+// agree).  256^3, trace+gather per component through L1: tricubic 1.76 -> 1.52,
+// triquintic staged 3.29 -> 3.12 ms.
 __device__ __forceinline__ int half_cell(const SlcParams &P, double z)
 {
     if (P.zbin) {
