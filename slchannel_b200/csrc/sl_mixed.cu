@@ -122,6 +122,21 @@ __device__ __forceinline__ float tri32(MixedView V, int i0, int i1, float tx, in
     return fl + dot2f(wz0, __ldg(V.mean32 + k0), wz1, __ldg(V.mean32 + k0 + 1));
 }
 
+// The FP64 plane mean m at a foot from its FP32 z weights, which sum to 1: the
+// middle node's value plus the weighted differences from it.  Summing wz m
+// itself multiplies the weights' rounding (6e-8) by the whole mean; here it
+// multiplies what the mean changes by across the stencil.
+template <int O>
+__device__ __forceinline__ double mean_at(const double *__restrict__ m, const float (&wz)[O])
+{
+    const double r = __ldg(m + O / 2 - 1);
+    double d = 0.0;
+#pragma unroll
+    for (int k = 0; k < O; ++k)
+        if (k != O / 2 - 1) d = fma((double)wz[k], __ldg(m + k) - r, d);
+    return r + d;
+}
+
 // Trajectory velocity at arrival + (ddx, ddy) (index units) and height
 // za + dz.  Heights enter the weights as differences formed in FP64 (an FP32
 // absolute height near z = Lz would carry ~1e-7 absolute error, a sizeable
@@ -248,10 +263,7 @@ __device__ __forceinline__ double gather_foot32(const SlcParams &P, MixedView F,
         for (int k = 0; k < O; ++k) m = fmaf(st.wz[k], __ldg(F.mean32 + k0 + k), m);
         return (double)(acc + m);
     }
-    double mean = 0.0;
-#pragma unroll
-    for (int k = 0; k < O; ++k) mean = fma((double)st.wz[k], __ldg(F.mean + k0 + k), mean);
-    return (double)acc + mean;
+    return (double)acc + mean_at<O>(F.mean + k0, st.wz);
 }
 
 // The trajectory velocity with tricubic Lagrange sampling (traj_interp_order
@@ -508,10 +520,7 @@ __device__ __forceinline__ double gather_box_m32(const SlcParams &P, const Mixed
         acc = fmaf(wx[i], accy, acc);
     }
 #endif
-    double mean = 0.0;
-#pragma unroll
-    for (int k = 0; k < O; ++k) mean = fma((double)wz[k], __ldg(F.mean + f.k0 + k), mean);
-    return (double)acc + mean;
+    return (double)acc + mean_at<O>(F.mean + f.k0, wz);
 }
 
 
