@@ -70,12 +70,14 @@ static_assert((kBX * sizeof(double)) % 128 == 0, "box rows of whole bank cycles"
 __host__ __device__ inline int padded_nx(int nx) { return (nx + kBX + 1) & ~1; }
 __host__ __device__ inline int padded_ny(int ny) { return ny + kBY; }
 
-// Unwrapped stencil base of one coordinate relative to the tile origin
-// (NaN or far-out values give a large sentinel that no box fits).
+// Unwrapped stencil base of one coordinate relative to the tile origin; NaN and
+// bases 4096 cells or more away give kFar, which box_fits refuses (the wrapping
+// L1 gather serves such feet).
+constexpr int kFar = 1 << 20;
 __device__ __forceinline__ int rel_base(double f, int h, int origin)
 {
     const double r = f - (double)h - (double)origin;
-    if (!(r > -4096.0 && r < 4096.0)) return 1 << 20;
+    if (!(r > -4096.0 && r < 4096.0)) return kFar;
     return (int)r;
 }
 
@@ -187,7 +189,7 @@ __device__ __forceinline__ bool box_fits(const int *r, int i0, int j0, const Slc
                                          int &Z0, int &ox)
 {
     const bool fit = r[0] <= r[1] && r[1] - r[0] + O + 1 <= Box<O>::X && r[3] - r[2] + O <= Box<O>::Y &&
-                     r[5] - r[4] + O <= Box<O>::Z;
+                     r[5] - r[4] + O <= Box<O>::Z && r[1] < kFar && r[3] < kFar;
     X0 = Y0 = Z0 = ox = 0;
     if (fit) {
         X0 = (i0 + r[0]) % P.nx;

@@ -91,3 +91,32 @@ def test_staged_on_a_shallow_grid_is_the_l1_path():
         assert torch.equal(x, y)
     assert na == nb
     assert _both(f, 0.05)[1][1] == 0
+
+
+@pytest.mark.parametrize("order", [6, 4])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_staged_equals_l1_thousands_of_cells_away(axis, order):
+    """A uniform U* moving every foot by 5000.37 cells, so that all of a block's
+    feet lie beyond the range the box search tells apart: V^n = U0 + a and
+    V^{n-1} = U0 + 2 a with a random a."""
+    f = _flow((64, 32, 40), 0.01, 0.1, order)
+    g = torch.Generator().manual_seed(4)
+    a = [0.1 * torch.randn(t.shape, generator=g, dtype=torch.float64).to(t.device) for t in (f.u, f.v, f.w)]
+    cells, step = 5000.37, (f.dx, f.dy)[axis]
+    for scale in (2.0, 1.0):  # V^{n-1}, then V^n
+        for c, (t, r) in enumerate(zip((f.u, f.v, f.w), a)):
+            t.copy_(scale * r)
+            if c == axis:
+                t += 1.0
+            if c == 2:  # no flow through the walls
+                t[:, :, 0] = 0.0
+                t[:, :, -1] = 0.0
+        f.apply_bc_uvw()
+        if scale == 2.0:
+            prev = [t.clone() for t in (f.u, f.v, f.w)]
+    for t, p in zip((f.u_nm1, f.v_nm1, f.w_nm1), prev):
+        t.copy_(p)
+    (x, nx), (y, ny) = _both(f, cells * step)[0]
+    for c, p, q in zip("uvw", x, y):
+        assert torch.isfinite(p).all() and torch.equal(p, q), c
+    assert nx == ny
