@@ -1227,13 +1227,8 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
     // 4. SL predictor: U* recomputed
     V3 M;
     if (mode == 2) {
-        for (int c = 0; c < 3; ++c)
-            if (!g->mid[c]) {
-                void *q = nullptr;
-                ADJ_CK(cudaMalloc(&q, g->ghost_elems[c] * sizeof(double)), "U* workspace");
-                g->allocs.push_back(q);
-                g->mid[c] = (double *)q;
-            }
+        rc = slc_grid_ensure_mid(g);
+        if (rc) return rc;
         ADJ_CK(launch_star(Tri{cur[0], cur[1], cur[2]}, Tri{prev[0], prev[1], prev[2]},
                            TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->ghost_elems, s),
                "U*");

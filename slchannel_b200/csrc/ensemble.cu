@@ -494,16 +494,14 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
         for (int l = 0; l < 3; ++l)
             for (int c = 0; c < 3; ++c) I.lev[l][c] = lev[i * 9 + l * 3 + c];
         I.p = p[i];
-        for (int c = 0; c < 3; ++c) {
-            if (!g->mid[c]) {
-                void *q = nullptr;
-                ENS_CK(cudaMalloc(&q, g->ghost_elems[c] * sizeof(double)), "U* workspace");
-                g->allocs.push_back(q);
-                g->mid[c] = (double *)q;
-                ENS_CK(cudaMemset(q, 0, g->ghost_elems[c] * sizeof(double)), "memset");
-            }
-            I.mid[c] = g->mid[c];
+        if (!g->mid[0]) {
+            const int rm = slc_grid_ensure_mid(g);
+            if (rm) return efail(e, rm, std::string("instance ") + std::to_string(i) + ": " + g->err);
+            // autotune also times instances whose U* the step keeps elsewhere
+            for (int c = 0; c < 3; ++c)
+                ENS_CK(cudaMemset(g->mid[c], 0, g->ghost_elems[c] * sizeof(double)), "memset");
         }
+        for (int c = 0; c < 3; ++c) I.mid[c] = g->mid[c];
         I.dzf = g->dzf;
         I.dzc = g->dzc;
         I.kx2 = g->kx2;
@@ -553,7 +551,7 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
             if (rs) return efail(e, rs, std::string("instance ") + std::to_string(i) + ": " + e->grids[i]->err);
             e->staged[i] = ready ? 1 : 0;
         }
-    ENS_CK(cudaDeviceSynchronize(), "z-solve tables");
+    ENS_CK(cudaDeviceSynchronize(), "z-solve tables and memsets");
     int rc = upload_tables(e);
     if (rc) return rc;
     e->bound = true;

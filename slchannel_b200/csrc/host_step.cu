@@ -225,7 +225,8 @@ int ensure_host_step(slc_grid *g)
             void *p = nullptr;
             HS_CK(cudaMalloc(&p, n * sizeof(double)), "host-step device state");
             g->allocs.push_back(p);
-            HS_CK(cudaMemset(p, 0, n * sizeof(double)), "memset");
+            // on the upload stream: every later use follows its copies or their events
+            HS_CK(cudaMemsetAsync(p, 0, n * sizeof(double), h->h2d), "memset");
             h->dev[s][q] = (double *)p;
         }
         void *p = nullptr;

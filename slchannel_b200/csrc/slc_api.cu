@@ -183,24 +183,17 @@ int do_project(slc_grid *g, double *u, double *v, double *w, double *p, double d
     return SLC_OK;
 }
 
+// U* workspace, uninitialised: every pass that fills it writes each node that
+// is read (one allocation: each costs a new handle's first call).
 int ensure_mid(slc_grid *g)
 {
-    if (!g->mid[0] && !g->mid[1] && !g->mid[2]) {  // one allocation: each costs a new handle's first call
-        double *p = nullptr;
-        const size_t n = g->ghost_elems[0] + g->ghost_elems[1] + g->ghost_elems[2];
-        int rc = dalloc(g, &p, n, "U* workspace");
-        if (rc) return rc;
-        SLC_CK(cudaMemset(p, 0, n * sizeof(double)), "memset");
-        g->mid[0] = p;
-        g->mid[1] = p + g->ghost_elems[0];
-        g->mid[2] = g->mid[1] + g->ghost_elems[1];
-    }
-    for (int c = 0; c < 3; ++c)
-        if (!g->mid[c]) {
-            int rc = dalloc(g, &g->mid[c], g->ghost_elems[c], "U* workspace");
-            if (rc) return rc;
-            SLC_CK(cudaMemset(g->mid[c], 0, g->ghost_elems[c] * sizeof(double)), "memset");
-        }
+    if (g->mid[0]) return SLC_OK;
+    double *p = nullptr;
+    const int rc = dalloc(g, &p, g->ghost_elems[0] + g->ghost_elems[1] + g->ghost_elems[2], "U* workspace");
+    if (rc) return rc;
+    g->mid[0] = p;
+    g->mid[1] = p + g->ghost_elems[0];
+    g->mid[2] = g->mid[1] + g->ghost_elems[1];
     return SLC_OK;
 }
 
@@ -244,8 +237,7 @@ int ensure_mixed_tma(slc_grid *g)
     float *p = nullptr;
     rc = dalloc(g, &p, off[6], "padded FP32 copies");
     if (rc) return rc;
-    SLC_CK(cudaMemset(p, 0, off[6] * sizeof(float)), "memset");
-    for (int q = 0; q < 6; ++q) g->tmx.pad[q] = p + off[q];
+    for (int q = 0; q < 6; ++q) g->tmx.pad[q] = p + off[q];  // the pack writes every entry
     if (mixed_tma_encode(g->P, g->mws, g->tmx) != cudaSuccess) {
         g->tmx_state = -1;
         return SLC_OK;
@@ -722,9 +714,7 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     CREATE_CK(dalloc(g, &g->th_id, 2 * ncplx, "Poisson elimination factors"));
     g->th_g = g->th_id + ncplx;
     {
-        // creation is synchronous: later work may come on any stream
         cudaError_t e = launch_thomas_factors(P, g->th_id, g->th_g, g->kx2, g->ky2, g->cl, g->cr, false, 0);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         if (e != cudaSuccess) {
             slc_grid_destroy(g);
             return fail(nullptr, SLC_E_CUDA, std::string("Poisson elimination factors: ") + cudaGetErrorString(e));
@@ -735,8 +725,10 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     CREATE_CK(dalloc(g, &g->scal, (size_t)8, "scalars"));
     CREATE_CK(dalloc(g, &g->dev_flags, (size_t)4, "device flags"));
     g->ticket = (unsigned *)(g->scal + 7);  // scal[0..1]: shift, forcing
+    // creation is synchronous: later work may come on any stream, and the uploads
+    // and memsets above (legacy stream) may still be under way on the device
     if (cudaMemset(g->dev_flags, 0, 4 * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemset(g->scal, 0, 8 * sizeof(double)) != cudaSuccess) {
+        cudaMemset(g->scal, 0, 8 * sizeof(double)) != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
         slc_grid_destroy(g);
         return fail(nullptr, SLC_E_CUDA, "memset device flags");
     }
@@ -1151,7 +1143,10 @@ int slc_gather_stats(slc_grid *g, int64_t *out4, int reset)
     unsigned long long h[4];
     SLC_CK(cudaMemcpy(h, g->dev_flags, sizeof(h), cudaMemcpyDeviceToHost), "read gather stats");
     for (int q = 0; q < 4; ++q) out4[q] = (int64_t)h[q];
-    if (reset) SLC_CK(cudaMemset(g->dev_flags, 0, sizeof(h)), "reset gather stats");
+    if (reset) {  // done before the caller's next launch on whatever stream
+        SLC_CK(cudaMemset(g->dev_flags, 0, sizeof(h)), "reset gather stats");
+        SLC_CK(cudaStreamSynchronize(0), "reset gather stats");
+    }
     return SLC_OK;
 }
 
