@@ -191,7 +191,8 @@ SLC_API int slc_host_step_stats(slc_grid *g, int64_t *out4);
  * slc_trace_gather_bdf2).  Results are bit-identical to
  * slc_trace_gather_bdf2's.  FP64 handles (nz >= 47 or nx >= 32): U* and the
  * padded copies are written with x fastest, and x runs along the lanes;
- * slc_step_bdf2 at order 6 gathers this way while the feet fit.  Mixed
+ * slc_step_bdf2 at order 6 gathers this way while the feet fit, on grids whose
+ * nx fills the lanes well enough for it to be the faster.  Mixed
  * handles (nz >= 62): FP32 fluctuation boxes, the padded copies written by
  * the mixed pack itself; slc_step_bdf2 on a mixed handle gathers this way.
  * slc_gather_stats reports how many boxes were staged.  Synchronous: it

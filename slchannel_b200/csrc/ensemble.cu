@@ -28,8 +28,8 @@ struct slc_ensemble {
     std::vector<slc_grid *> grids;
     std::vector<EnsInst> host_inst;
     std::vector<int> tkl;
-    // instances whose trace+gather runs as the single-grid TMA-staged launches
-    // (large enough to fill the GPU alone) instead of in the persistent kernel
+    // instances whose trace+gather runs as single-grid launches (large enough to
+    // fill the GPU alone) instead of in the persistent kernel
     std::vector<char> staged;
     bool bound = false;
     std::string err;
@@ -60,13 +60,17 @@ struct slc_ensemble {
     cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
 };
 
-// An order-6 instance whose staged trace+gather has at least this many
-// blocks per component (a few waves of the GPU) runs it as its own launches.
-// It gathers from boxes while the mean flow moves less than this many cells per
-// step, through L1 alone above: the boxes leave three cells of spread in y and z,
-// which the fluctuations of a flow that moves further exceed in many blocks
-// (128x64x128 at 1.8 cells: a third of the far boxes; staged 3.5 ms, L1 2.6 ms
-// for the three such instances of the 12-channel benchmark ensemble).
+// An order-6 instance whose trace+gather has at least this many blocks per
+// component (a few waves of the GPU) runs it as its own launches: an FP64 one
+// with x along the lanes where that pays (tma_pays), else k_sl (three of
+// 128x128x128 with tricubic trajectories: 9.5 ms a step, 10.9 in the persistent
+// kernel; of 40x128x128: 1.60 ms, 1.73 there, 1.85 with x along the lanes).
+// With x along the lanes it gathers from boxes while the mean flow moves less
+// than kEnsBoxCells cells per step, through L1 alone above: the boxes leave three
+// cells of spread in y and z, which the fluctuations of a flow that moves further
+// exceed in many blocks (128x64x128 at 1.8 cells: a third of the far boxes; staged
+// 3.5 ms, L1 2.6 ms for the three such instances of the 12-channel benchmark
+// ensemble).
 constexpr double kEnsBoxCells = 1.5;
 #ifndef SLC_ENS_STAGED_MIN_BLOCKS
 #define SLC_ENS_STAGED_MIN_BLOCKS 2048
@@ -141,12 +145,15 @@ void free_groups(slc_ensemble *e)
         }
 }
 
-// Blocks per component of an instance's staged trace+gather.
+// Blocks per component of an instance's own trace+gather launches.
 long long staged_blocks(const SlcParams &P, bool mixed)
 {
     if (mixed) return (long long)((P.nz + 31) / 32) * ((P.ny + 3) / 4) * ((P.nx + 1) / 2);
     return (long long)((P.nx + 31) / 32) * ((P.ny + 1) / 2) * ((P.nz + 3) / 4);
 }
+
+// Whether an FP64 instance's own launches gather from boxes.
+bool ens_boxes(const EnsInst &H) { return H.dt * H.U_bulk * H.P.inv_dx < kEnsBoxCells; }
 
 // Work items of every multi-instance kernel, in one array.
 void build_items(slc_ensemble *e, std::vector<EnsItem> &items)
@@ -311,11 +318,16 @@ int enqueue_step(slc_ensemble *e, int ph, cudaStream_t s)
                    "mixed-form pack (padded)");
             ENS_CK(launch_sl_mixed_tma(g->P, a, b, g->mws, g->tmx, H.dt, o, H.ncl, g->dev_flags, s),
                    "mixed trace+gather BDF2 (TMA-staged)");
+        } else if (g->tma_state != 1 || !tma_pays(g->P, ens_boxes(H))) {
+            ENS_CK(launch_star(a, b, TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->ghost_elems, s),
+                   "U* = 2V^n - V^{n-1}");
+            ENS_CK(launch_sl(g->P, 2, a, b, Tri{g->mid[0], g->mid[1], g->mid[2]}, false, H.dt, o, H.ncl, s),
+                   "trace+gather BDF2");
         } else {
             ENS_CK(launch_mid_pack(g->P, a, b, TriMut{g->mid[0], g->mid[1], g->mid[2]}, g->tma, s),
                    "U* and padded node copies");
             ENS_CK(launch_sl_tma(g->P, Tri{g->mid[0], g->mid[1], g->mid[2]}, H.dt, o, H.ncl, g->dev_flags,
-                                 g->tma, H.dt * H.U_bulk * g->P.inv_dx < kEnsBoxCells, s),
+                                 g->tma, ens_boxes(H), s),
                    "trace+gather BDF2 (TMA-staged)");
         }
     }
@@ -538,14 +550,18 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
             I.mws = g->mws;
         }
     }
-    // the large order-6 instances gather through the single-grid staged
-    // launches (each fills the GPU alone); the rest share the persistent kernel
+    // the large order-6 instances gather through single-grid launches (each
+    // fills the GPU alone); the rest share the persistent kernel
     e->staged.assign(n, 0);
     if (e->order == 6)
         for (int i = 0; i < n; ++i) {
             const SlcParams &P = e->grids[i]->P;
             const long long blocks = staged_blocks(P, e->mixed);
             if (blocks < SLC_ENS_STAGED_MIN_BLOCKS) continue;
+            if (!e->mixed && !tma_pays(P, ens_boxes(e->host_inst[i]))) {
+                e->staged[i] = 1;  // k_sl
+                continue;
+            }
             bool ready = false;
             int rs = slc_grid_ensure_staged(e->grids[i], &ready);
             if (rs) return efail(e, rs, std::string("instance ") + std::to_string(i) + ": " + e->grids[i]->err);

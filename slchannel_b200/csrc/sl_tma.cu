@@ -204,9 +204,11 @@ __device__ __forceinline__ bool box_fits(const int *r, int i0, int j0, const Slc
 }
 
 // VN, VM: the padded copies of V^n and V^{n-1}.  TO, NI: trajectory order and
-// iterations (2, 2), or 0, 0 to read them from P.
+// iterations, 0 to read them from P.  Tricubic trajectories take two blocks' 128
+// registers (step at 96x96x96: 1.42 ms at two blocks, 1.47 at three, 1.50 at four;
+// 1.63 with k_sl).
 template <int C, int O, int TO, int NI>
-__global__ void __launch_bounds__(kThreads, Box<O>::min_blocks)
+__global__ void __launch_bounds__(kThreads, TO == 4 ? 2 : Box<O>::min_blocks)
     k_sl_tma(const __grid_constant__ SlcParams P, const __grid_constant__ Vel3X M, const __grid_constant__ NodeViewX VN,
              const __grid_constant__ NodeViewX VM, double dt, double *__restrict__ out, unsigned long long *nclamp,
              unsigned long long *stats, const __grid_constant__ CUtensorMap tmN,
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, Box<O>::min_blocks)
 }
 
 // The same through L1 alone, for order-6 flows whose feet spread wider than a
-// box: no barriers, and 128 registers for the weights.  Three instances of the
+// box (where tma_pays says so): no barriers, and 128 registers for the weights.  Three instances of the
 // 12-channel ensemble at 1.8 cells of mean displacement a step: 2.57 ms, against
 // 3.5 ms with boxes (a third to three quarters of the far ones do not fit) and
 // 3.03 ms with boxes and z along the lanes.  At order 4 k_sl is faster (256^3:
@@ -446,13 +448,43 @@ cudaError_t launch_tma_t(const SlcParams &P, const Vel3X &M, double dt, TriMut o
 
 }  // namespace
 
-// Boxes fit inside the padded arrays in every dimension, and enough lanes find
-// a point: shallow and narrow grids (nz < 47 and nx < 32) stay with k_sl, as do
-// grids whose padded copies exceed 32-bit indices or a launch grid's y extent.
+// Boxes fit inside the padded arrays in every dimension; shallow and narrow
+// grids (nz < 47 and nx < 32) have none, nor do grids whose padded copies exceed
+// 32-bit indices or a launch grid's y extent.
 bool tma_supported(const SlcParams &P)
 {
     if (P.ny > 60000 || (double)(P.nx + kBX + 1) * padded_ny(P.ny) * (P.nz + 2) >= 2147483647.0) return false;
     return P.nz + 1 >= kBZ && (P.nz + 1 >= 48 || P.nx >= 32) && encode_fn() != nullptr;
+}
+
+// Whether a triquintic step is faster with x along the lanes than with k_sl
+// (z along the lanes): from boxes, or through L1 where the feet spread too far.
+// Whole steps, x lanes / k_sl, on a B200:
+// - Lanes past the last x are idle and the copies are 48 nodes wider than the
+//   grid.  Boxes, ny = nz = 128: 1.50 at nx 16, 1.29 at 24, 1.04 at 32, 1.33 at 33,
+//   1.14 at 40, 0.98 at 48, 0.82 at 64, 1.06 at 65, 0.97 at 72; 256x128x128 0.75.
+//   So three quarters of the lanes, from nx = 32.  A launch of less than one
+//   wave hardly feels idle lanes (24x16x48 1.08, and 0.66 of what it took from
+//   boxes with z along the lanes): there from nx = 24.
+// - Through L1, k_sl's lanes spread with the profile over 32 levels, all of
+//   it at nz = 32: 0.83 on 64x64x32, 0.85 on 128x96x64, 0.92 on 96x96x96, but 1.09
+//   on 64x128x128, 1.31 on 97x128x128, 1.02 on 120x120x120, 0.97 on 128x128x128.
+//   Up to 32 levels fewer lanes do (64x32 in y and z): from boxes 0.88 at nx 44,
+//   0.95 at 65, 1.04 at 33; through L1 0.87 at 48, 0.90 at 72, 0.97 at 44, 1.04 at 65.
+// - Tricubic trajectories read 64 nodes per sample through L1, so the same line
+//   as without boxes: 0.88 on 96x96x96, 0.84 on 192x128x96, 0.72 on 192x96x32, 0.97
+//   on 256x192x192, but 1.04 on 80x64x96, 1.03 on 97x75x81, 1.02 on 64x128x128; two
+//   iterations (unrolled, else 1.09 on 128x128x128).
+bool tma_pays(const SlcParams &P, bool staged)
+{
+    const int tiles = (P.nx + kTI - 1) / kTI;
+    const double lanes = (double)P.nx / (kTI * tiles);
+    const bool shallow = P.nz <= 32, cubic = P.traj_order != 2;
+    if (cubic && P.n_iters != 2) return false;
+    if (!staged || cubic)
+        return P.nx >= kTI && (P.nz <= 96 ? lanes >= (shallow ? 0.75 : 0.875) : P.nx >= 96 && lanes >= 0.96);
+    const long long blocks = 3LL * tiles * ((P.ny + kTJ - 1) / kTJ) * ((P.nz + kTK - 1) / kTK);
+    return lanes >= (shallow ? 0.65 : 0.75) && (P.nx >= kTI || blocks <= 148 * Box<6>::min_blocks);
 }
 
 size_t tma_padded_elems(const SlcParams &P, int comp)
@@ -509,8 +541,9 @@ cudaError_t launch_sl_tma(const SlcParams &P, Tri mid, double dt, TriMut out, un
     if (P.order == 4)
         return usual ? launch_tma_t<4, 2, 2>(P, M, dt, out, nclamp, stats, T, staged, s)
                      : launch_tma_t<4, 0, 0>(P, M, dt, out, nclamp, stats, T, staged, s);
-    return usual ? launch_tma_t<6, 2, 2>(P, M, dt, out, nclamp, stats, T, staged, s)
-                 : launch_tma_t<6, 0, 0>(P, M, dt, out, nclamp, stats, T, staged, s);
+    if (usual) return launch_tma_t<6, 2, 2>(P, M, dt, out, nclamp, stats, T, staged, s);
+    if (P.n_iters == 2) return launch_tma_t<6, 4, 2>(P, M, dt, out, nclamp, stats, T, staged, s);
+    return launch_tma_t<6, 0, 0>(P, M, dt, out, nclamp, stats, T, staged, s);
 }
 
 // One 3-D tiled tensor map (z innermost, no swizzle, zero fill) over a node

@@ -353,9 +353,9 @@ enum GatherMode { kGatherDefault, kGatherL1, kGatherStaged };
 #endif
 // The step keeps gathering from staged boxes while at least this fraction of
 // the blocks staged both feet, and otherwise gathers through L1 (whose
-// kernel holds more registers per thread, so it is the faster when many
+// kernels hold more registers per thread, so they are the faster when many
 // blocks would fall back), trying the staged gather again every
-// kStagedProbeEvery calls.  The two gathers give the same results.
+// kStagedProbeEvery calls.  All of them give the same results.
 constexpr double kStagedMinFraction = 0.9;
 constexpr int kStagedProbeEvery = 50;
 
@@ -458,15 +458,18 @@ int do_trace_gather_bdf2(slc_grid *g, const double *const cur[3], const double *
         tim_end(g, t, s);
         return SLC_OK;
     }
-    // By default an order-6 step reads the fields through copies with x fastest,
-    // from boxes while the feet fit them (choose_staged), else through L1 alone;
-    // order 4 keeps k_sl (64 loads per foot leave too little to save).
-    const bool copies = mode == kGatherStaged || (mode == kGatherDefault && g->P.order == 6);
+    // By default an order-6 step reads the fields through copies with x fastest
+    // where that pays (tma_pays): from boxes while the feet fit them
+    // (choose_staged), else through L1 or with k_sl; order 4 keeps k_sl (64 loads
+    // per foot leave too little to save).
+    const bool forced = mode == kGatherStaged;
+    const bool copies = forced || (mode == kGatherDefault && g->P.order == 6 && tma_pays(g->P, true));
     int rc = ensure_mid(g);
     if (!rc && copies) rc = ensure_tma(g);
     if (rc) return rc;
-    const bool by_x = copies && g->tma_state == 1;
-    const bool staged = by_x && (mode == kGatherStaged || choose_staged(g, s));
+    const bool ready = copies && g->tma_state == 1;
+    const bool staged = ready && (forced || choose_staged(g, s));
+    const bool by_x = staged || (ready && tma_pays(g->P, false));
     if (by_x) {
         long t = tim_begin(g, SLC_PHASE_MID, s);
         SLC_CK(launch_mid_pack(g->P, Tri{cur[0], cur[1], cur[2]}, Tri{prev[0], prev[1], prev[2]},

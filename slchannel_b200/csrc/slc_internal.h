@@ -242,6 +242,7 @@ struct TmaSL {
 };
 size_t tma_padded_elems(const SlcParams &P, int comp);
 bool tma_supported(const SlcParams &P);
+bool tma_pays(const SlcParams &P, bool staged);  // against k_sl, from boxes or through L1
 cudaError_t tma_encode(const SlcParams &P, TmaSL &T);
 // U* (nodes with x fastest, in the mid arrays) and the padded copies.
 cudaError_t launch_mid_pack(const SlcParams &P, Tri cur, Tri prev, TriMut mid, const TmaSL &T,
