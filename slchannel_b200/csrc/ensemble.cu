@@ -13,6 +13,7 @@
 #include <cufft.h>
 
 #include <algorithm>
+#include <cmath>
 #include <map>
 #include <string>
 #include <utility>
@@ -66,7 +67,7 @@ struct slc_ensemble {
 // 128x128x128 with tricubic trajectories: 9.5 ms a step, 10.9 in the persistent
 // kernel; of 40x128x128: 1.60 ms, 1.73 there, 1.85 with x along the lanes).
 // With x along the lanes it gathers from boxes while the mean flow moves less
-// than kEnsBoxCells cells per step, through L1 alone above: the boxes leave three
+// than kEnsBoxCells cells per step either way, through L1 alone above: the boxes leave three
 // cells of spread in y and z, which the fluctuations of a flow that moves further
 // exceed in many blocks (128x64x128 at 1.8 cells: a third of the far boxes; staged
 // 3.5 ms, L1 2.6 ms for the three such instances of the 12-channel benchmark
@@ -153,7 +154,7 @@ long long staged_blocks(const SlcParams &P, bool mixed)
 }
 
 // Whether an FP64 instance's own launches gather from boxes.
-bool ens_boxes(const EnsInst &H) { return H.dt * H.U_bulk * H.P.inv_dx < kEnsBoxCells; }
+bool ens_boxes(const EnsInst &H) { return H.dt * std::fabs(H.U_bulk) * H.P.inv_dx < kEnsBoxCells; }
 
 // Work items of every multi-instance kernel, in one array.
 void build_items(slc_ensemble *e, std::vector<EnsItem> &items)

@@ -117,3 +117,16 @@ def test_ensemble_of_large_instances_equals_its_channels(n3, traj, dt):
     for i, f in enumerate(flows):
         for a, b in zip((*ens.velocity(i), ens.p[i]), (f.u, f.v, f.w, f.p)):
             assert float((a - b).abs().max()) <= 1e-12 * max(1.0, float(b.abs().max()))
+
+
+@pytest.mark.parametrize("direction", [1.0, -1.0])
+def test_ensemble_leaves_the_boxes_for_fast_mean_flow_either_way(direction):
+    """At 1.5 cells of mean displacement a step a large instance gathers through
+    L1, whichever way its flow goes."""
+    for dt, boxes in ((0.05, True), (0.2, False)):  # 0.76 and 3.06 cells
+        f = _flow((96, 64, 96), dt, direction=direction)
+        ens = ChannelEnsemble([f], [dt], autotune=False)
+        ens.step()
+        torch.cuda.synchronize()
+        handle = ctypes.c_void_p(N.lib().slc_ensemble_grid(ens._h, 0))
+        assert (_blocks(handle) > 0) == boxes
