@@ -909,7 +909,7 @@ struct AdjWS {
     int *sums = nullptr, *total = nullptr;
     double *lam_mid[3] = {nullptr, nullptr, nullptr};
     double *zs_tab = nullptr, zs_dt = 0.0;  // z-solve tables of the transposed systems, at zs_dt
-    double *th_id = nullptr, *th_g = nullptr;  // Poisson factors of the transposed systems
+    double *th_id = nullptr;  // Poisson inverse pivots of the transposed systems
     double *partials = nullptr, *S = nullptr;
     double *W = nullptr;  // sorted gather weights, 3 O arrays of n_c[0]
     int *kz = nullptr;    // sorted gather records' first z node
@@ -977,16 +977,15 @@ int ensure_adj(slc_grid *g, cudaStream_t s)
     if (!rc) rc = adj_alloc(g, &w->kz, (size_t)w->n_c[0], "adjoint gather z bases");
     if (!rc) rc = adj_alloc(g, &w->part, (size_t)8 * w->nkeys_max, "adjoint partial sums");
     const size_t ncplx = (size_t)P.nz * P.nx * (P.ny / 2 + 1);
-    if (!rc) rc = adj_alloc(g, &w->th_id, ncplx, "adjoint Poisson factors");
-    if (!rc) rc = adj_alloc(g, &w->th_g, ncplx, "adjoint Poisson factors");
+    if (!rc) rc = adj_alloc(g, &w->th_id, ncplx, "adjoint Poisson inverse pivots");
     if (rc) {
         delete w;
         return rc;
     }
-    cudaError_t e = launch_thomas_factors(P, w->th_id, w->th_g, g->kx2, g->ky2, g->cl, g->cr, true, s);
+    cudaError_t e = launch_thomas_factors(P, w->th_id, g->kx2, g->ky2, g->cl, g->cr, true, s);
     if (e != cudaSuccess) {
         delete w;
-        g->err = std::string("adjoint Poisson factors: ") + cudaGetErrorString(e);
+        g->err = std::string("adjoint Poisson inverse pivots: ") + cudaGetErrorString(e);
         return SLC_E_CUDA;
     }
     g->adj = w;
@@ -1207,7 +1206,7 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
         g->err = "cufftExecD2Z (adjoint)";
         return SLC_E_CUFFT;
     }
-    ADJ_CK(launch_thomas_poisson(P, g->hat, w->th_id, w->th_g, g->cl, g->cr, s, true), "Poisson Thomas adjoint");
+    ADJ_CK(launch_thomas_poisson(P, g->hat, w->th_id, g->cl, g->cr, s, true), "Poisson Thomas adjoint");
     if (cufftSetStream(g->inv, s) != CUFFT_SUCCESS ||
         cufftExecZ2D(g->inv, (cufftDoubleComplex *)g->hat, g->rhs) != CUFFT_SUCCESS) {
         g->err = "cufftExecZ2D (adjoint)";

@@ -524,8 +524,9 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
         const slc_ensemble::Group &gr = e->groups[group_of[i]];
         I.rhs = gr.rhs + (size_t)plane_off[i] * P.nx * P.ny;
         I.hat = gr.hat + (size_t)2 * plane_off[i] * P.nx * (P.ny / 2 + 1);
+        const int rp = slc_grid_ensure_pivots(g, 0);
+        if (rp) return efail(e, rp, std::string("instance ") + std::to_string(i) + ": " + g->err);
         I.th_id = g->th_id;
-        I.th_g = g->th_g;
         double *tab = nullptr;
         int rc = ealloc(e, &tab, zsolve_table_doubles(P.nz), "z-solve tables");
         if (rc) return rc;
@@ -568,7 +569,7 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
             if (rs) return efail(e, rs, std::string("instance ") + std::to_string(i) + ": " + e->grids[i]->err);
             e->staged[i] = ready ? 1 : 0;
         }
-    ENS_CK(cudaDeviceSynchronize(), "z-solve tables and memsets");
+    ENS_CK(cudaDeviceSynchronize(), "tables and memsets");
     int rc = upload_tables(e);
     if (rc) return rc;
     e->bound = true;

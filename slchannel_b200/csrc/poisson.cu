@@ -201,19 +201,19 @@ __device__ __forceinline__ Row3 poisson_row(const double *__restrict__ cl, const
 // Twisted (two-ended) Thomas elimination.  Half 0 eliminates rows 0 .. m-1
 // downwards as the reference's Thomas sweep does; half 1 eliminates rows
 // nz-1 .. m+1 upwards (sub- and super-diagonal exchanged); the two meet at row
-// m = nz/2, and each back-substitutes its half.  The factors depend on the grid
-// alone: k_thomas_factors computes them once per handle (row k of column col at
-// k * ncol + col: th_id the inverse pivots, the meeting row's included, th_g the
-// pivot ratios).  A sweep then has two dependent operations per row where
-// dividing by the pivot on the way was a chain of some thirty: 12.2 -> 6.3 us
-// at 32^3, 24 -> 12 us at 64^3, 211 -> 109 us at 256^3 (0.7 GB: bound there by the
-// traffic, which the table leaves as it was: one word read where a pivot ratio
-// was stored).  The table alone, with the loads of a row still tested one by one
-// behind the chain, was no faster at 64^3 (29 us): the batches below matter as
-// much.
+// m = nz/2, and each back-substitutes its half.  The inverse pivots depend on the
+// grid alone: k_thomas_factors computes them once per handle, at its first
+// projection (row k of column col at k * ncol + col, the meeting row's included).
+// A row's pivot ratio is its outward coupling times its inverse pivot, so the one
+// table serves both halves of a sweep.  A sweep then has two dependent operations
+// per row where dividing by the pivot on the way was a chain of some thirty:
+// 12.2 -> 6.3 us at 32^3, 24 -> 12 us at 64^3, 211 -> 109 us at 256^3 (0.7 GB: bound
+// there by the traffic, which the table leaves as it was: one word read where a
+// pivot ratio was stored).  The table alone, with the loads of a row still tested
+// one by one behind the chain, was no faster at 64^3 (29 us): the batches below
+// matter as much.
 template <bool T>
 __global__ void __launch_bounds__(256) k_thomas_factors(SlcParams P, double *__restrict__ th_id,
-                                                        double *__restrict__ th_g,
                                                         const double *__restrict__ kx2,
                                                         const double *__restrict__ ky2,
                                                         const double *__restrict__ cl,
@@ -233,18 +233,15 @@ __global__ void __launch_bounds__(256) k_thomas_factors(SlcParams P, double *__r
         const double id = 1.0 / (R.b - R.a * gt);
         gt = R.c * id;
         th_id[(size_t)k * ncol + col] = id;
-        th_g[(size_t)k * ncol + col] = gt;
     }
     for (int k = nz - 1; k > m; --k) {
         const Row3 R = poisson_row<T>(cl, cr, k2, nz, k, pinned);
         const double id = 1.0 / (R.b - R.c * gb);
         gb = R.a * id;
         th_id[(size_t)k * ncol + col] = id;
-        th_g[(size_t)k * ncol + col] = gb;
     }
     const Row3 R = poisson_row<T>(cl, cr, k2, nz, m, pinned);
     th_id[(size_t)m * ncol + col] = 1.0 / (R.b - R.a * gt - R.c * gb);
-    th_g[(size_t)m * ncol + col] = 0.0;
 }
 
 // The sweep: four threads per column, part (re / im) x half, the halves of a
@@ -267,8 +264,7 @@ __device__ __forceinline__ void thomas_coef(const SlcParams &P, const double *__
 
 template <bool T = false>
 __device__ __forceinline__ void thomas_column(const SlcParams &P, double *__restrict__ hat,
-                                              const double *__restrict__ th_id,
-                                              const double *__restrict__ th_g, const double *coef, double norm,
+                                              const double *__restrict__ th_id, const double *coef, double norm,
                                               int t)
 {
     const int nky = P.ny / 2 + 1;
@@ -278,7 +274,7 @@ __device__ __forceinline__ void thomas_column(const SlcParams &P, double *__rest
     const int nz = P.nz, m = nz / 2;
     const size_t st = 2 * (size_t)ncol, sf = (size_t)ncol;  // doubles per k-plane: spectrum, factors
     double *h = hat + 2 * (size_t)(active ? col : 0) + part;
-    const double *id = th_id + (active ? col : 0), *g = th_g + (active ? col : 0);
+    const double *id = th_id + (active ? col : 0);
     const int cnt = active ? (half ? nz - 1 - m : m) : 0;  // rows this thread eliminates
     const int last = max(cnt - 1, 0);
     // the pinned mode's row 0 (transposed: row 1) lacks one coupling
@@ -327,7 +323,7 @@ __device__ __forceinline__ void thomas_column(const SlcParams &P, double *__rest
     for (int u = 0; u < kPre; ++u) {
         const int k = back(min(u, last));
         dn[u] = h[k * st];
-        fn[u] = __ldg(g + k * sf);
+        fn[u] = __ldg(id + k * sf);
     }
     __syncwarp();  // every lane has read row m before the top half writes it
     if (active && half == 0) h[m * st] = xm * norm;
@@ -342,13 +338,13 @@ __device__ __forceinline__ void thomas_column(const SlcParams &P, double *__rest
         for (int u = 0; u < kPre; ++u) {
             const int k = back(min(q0 + kPre + u, last));
             dn[u] = h[k * st];
-            fn[u] = __ldg(g + k * sf);
+            fn[u] = __ldg(id + k * sf);
         }
 #pragma unroll
         for (int u = 0; u < kPre; ++u) {
-            const int q = q0 + u;
-            x = d[u] - f[u] * x;
-            if (q < cnt) h[back(q) * st] = x * norm;
+            const int q = q0 + u, k = back(min(q, last));
+            x = d[u] - (half ? down(k) : up(k)) * f[u] * x;
+            if (q < cnt) h[k * st] = x * norm;
         }
     }
 }
@@ -358,13 +354,12 @@ constexpr int kThomasT = 64;  // small blocks: a 64^3 spectrum's columns still r
 template <bool T>
 __global__ void __launch_bounds__(kThomasT) k_thomas(SlcParams P, double *__restrict__ hat,
                                                      const double *__restrict__ th_id,
-                                                     const double *__restrict__ th_g,
                                                      const double *__restrict__ cl,
                                                      const double *__restrict__ cr, double norm)
 {
     extern __shared__ double coef[];
     thomas_coef<T>(P, cl, cr, coef);
-    thomas_column<T>(P, hat, th_id, th_g, coef, norm, blockIdx.x * blockDim.x + threadIdx.x);
+    thomas_column<T>(P, hat, th_id, coef, norm, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // --------------------------------------------------------------------------
@@ -616,7 +611,7 @@ __global__ void __launch_bounds__(kThomasT) k_thomas_ens(const EnsInst *__restri
     const double norm = 1.0 / ((double)I.P.nx * (double)I.P.ny);
     extern __shared__ double coef[];
     thomas_coef<false>(I.P, I.cl, I.cr, coef);
-    thomas_column(I.P, I.hat, I.th_id, I.th_g, coef, norm,
+    thomas_column(I.P, I.hat, I.th_id, coef, norm,
                   it.a * blockDim.x + threadIdx.x);
 }
 
@@ -715,26 +710,26 @@ cudaError_t launch_divergence(const SlcParams &P, Tri f, const double *dz_f, dou
     return cudaGetLastError();
 }
 
-cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, double *th_g, const double *kx2,
-                                  const double *ky2, const double *cl, const double *cr, bool transposed,
+cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, const double *kx2, const double *ky2,
+                                  const double *cl, const double *cr, bool transposed,
                                   cudaStream_t s)
 {
     const unsigned nb = (unsigned)(((long long)P.nx * (P.ny / 2 + 1) + 255) / 256);
-    if (transposed) k_thomas_factors<true><<<nb, 256, 0, s>>>(P, th_id, th_g, kx2, ky2, cl, cr);
-    else k_thomas_factors<false><<<nb, 256, 0, s>>>(P, th_id, th_g, kx2, ky2, cl, cr);
+    if (transposed) k_thomas_factors<true><<<nb, 256, 0, s>>>(P, th_id, kx2, ky2, cl, cr);
+    else k_thomas_factors<false><<<nb, 256, 0, s>>>(P, th_id, kx2, ky2, cl, cr);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *th_g,
-                                  const double *cl, const double *cr, cudaStream_t s, bool transposed)
+cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *cl,
+                                  const double *cr, cudaStream_t s, bool transposed)
 {
     const long long nthr = 4LL * P.nx * (P.ny / 2 + 1);  // thomas_column: 4 per column
     const double norm = 1.0 / ((double)P.nx * (double)P.ny);
     const unsigned nb = (unsigned)((nthr + kThomasT - 1) / kThomasT);
     const size_t sm = 2 * (size_t)P.nz * sizeof(double);  // nz <= 1024
-    if (transposed) k_thomas<true><<<nb, kThomasT, sm, s>>>(P, hat, th_id, th_g, cl, cr, norm);
-    else k_thomas<false><<<nb, kThomasT, sm, s>>>(P, hat, th_id, th_g, cl, cr, norm);
+    if (transposed) k_thomas<true><<<nb, kThomasT, sm, s>>>(P, hat, th_id, cl, cr, norm);
+    else k_thomas<false><<<nb, kThomasT, sm, s>>>(P, hat, th_id, cl, cr, norm);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -151,6 +151,18 @@ int ensure_zsolve_tables(slc_grid *g, double dt, cudaStream_t s)
     return SLC_OK;
 }
 
+bool capturing(cudaStream_t s);
+
+// Poisson inverse pivots, at a handle's first projection (an advector's has
+// none).  A graph that captures it keeps the launch and refills the table.
+int ensure_pivots(slc_grid *g, cudaStream_t s)
+{
+    if (g->th_valid) return SLC_OK;
+    SLC_CK(launch_thomas_factors(g->P, g->th_id, g->kx2, g->ky2, g->cl, g->cr, false, s), "Poisson inverse pivots");
+    g->th_valid = !capturing(s);
+    return SLC_OK;
+}
+
 long tim_begin(slc_grid *g, int phase, cudaStream_t s);
 void tim_end(slc_grid *g, long slot, cudaStream_t s);
 
@@ -170,10 +182,12 @@ int do_project(slc_grid *g, double *u, double *v, double *w, double *p, double d
                double dt_proj, cudaStream_t s)
 {
     long t = tim_begin(g, SLC_PHASE_PROJECT, s);
+    int rc = ensure_pivots(g, s);
+    if (rc) return rc;
     SLC_CK(launch_div_pack(g->P, Tri{u, v, w}, g->dzf, dt_div, g->rhs, s), "divergence");
     SLC_FFT(cufftSetStream(g->fwd, s), "cufftSetStream");
     SLC_FFT(cufftExecD2Z(g->fwd, g->rhs, (cufftDoubleComplex *)g->hat), "cufftExecD2Z");
-    SLC_CK(launch_thomas_poisson(g->P, g->hat, g->th_id, g->th_g, g->cl, g->cr, s),
+    SLC_CK(launch_thomas_poisson(g->P, g->hat, g->th_id, g->cl, g->cr, s),
            "Poisson Thomas sweep");
     SLC_FFT(cufftSetStream(g->inv, s), "cufftSetStream");
     SLC_FFT(cufftExecZ2D(g->inv, (cufftDoubleComplex *)g->hat, g->rhs), "cufftExecZ2D");
@@ -276,6 +290,7 @@ int ensure_mixed(slc_grid *g)
 
 int slc_grid_ensure_mixed(slc_grid *g) { return ensure_mixed(g); }
 int slc_grid_ensure_mid(slc_grid *g) { return ensure_mid(g); }
+int slc_grid_ensure_pivots(slc_grid *g, cudaStream_t s) { return ensure_pivots(g, s); }
 
 int slc_grid_ensure_staged(slc_grid *g, bool *ready)
 {
@@ -714,15 +729,7 @@ int slc_grid_create(const slc_grid_desc *d, slc_grid **out)
     const size_t nreal = (size_t)nz * nx * ny, ncplx = (size_t)nz * nx * nky;
     CREATE_CK(dalloc(g, &g->rhs, nreal, "Poisson rhs"));
     CREATE_CK(dalloc(g, &g->hat, 2 * ncplx, "Poisson spectrum"));
-    CREATE_CK(dalloc(g, &g->th_id, 2 * ncplx, "Poisson elimination factors"));
-    g->th_g = g->th_id + ncplx;
-    {
-        cudaError_t e = launch_thomas_factors(P, g->th_id, g->th_g, g->kx2, g->ky2, g->cl, g->cr, false, 0);
-        if (e != cudaSuccess) {
-            slc_grid_destroy(g);
-            return fail(nullptr, SLC_E_CUDA, std::string("Poisson elimination factors: ") + cudaGetErrorString(e));
-        }
-    }
+    CREATE_CK(dalloc(g, &g->th_id, ncplx, "Poisson inverse pivots"));
     CREATE_CK(dalloc(g, &g->zs_tab, zsolve_table_doubles(nz), "z-solve tables"));
     CREATE_CK(dalloc(g, &g->partials, (size_t)kBulkBlocks, "bulk partials"));
     CREATE_CK(dalloc(g, &g->scal, (size_t)8, "scalars"));

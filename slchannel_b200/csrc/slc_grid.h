@@ -37,7 +37,9 @@ struct slc_grid {
     float *zc32 = nullptr, *zf32 = nullptr;
     float *dinv_c32[SLC_MAX_ORDER + 1] = {}, *dinv_f32[SLC_MAX_ORDER + 1] = {};
     double *kx2 = nullptr, *ky2 = nullptr, *cl = nullptr, *cr = nullptr;
-    double *rhs = nullptr, *hat = nullptr, *th_id = nullptr, *th_g = nullptr;
+    double *rhs = nullptr, *hat = nullptr;
+    double *th_id = nullptr;  // Poisson inverse pivots, filled at the first projection
+    bool th_valid = false;
     double *zs_tab = nullptr;
     double zs_dt = 0.0;
     bool zs_valid = false;
@@ -72,6 +74,8 @@ struct slc_grid {
 
 // Allocate the mixed form's workspace of a mixed-precision handle (slc_api.cu).
 int slc_grid_ensure_mixed(slc_grid *g);
+// Fill g->th_id on s if it is not yet (slc_api.cu).
+int slc_grid_ensure_pivots(slc_grid *g, cudaStream_t s);
 // Allocate the U* workspace g->mid (slc_api.cu).
 int slc_grid_ensure_mid(slc_grid *g);
 // Allocate what the handle's TMA-staged BDF2 gather needs (padded copies,

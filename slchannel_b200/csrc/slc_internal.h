@@ -111,13 +111,12 @@ cudaError_t launch_div_pack(const SlcParams &P, Tri f, const double *dz_f, doubl
                             double *rhs_zmajor, cudaStream_t s);
 cudaError_t launch_divergence(const SlcParams &P, Tri f, const double *dz_f, double *div,
                               cudaStream_t s);
-// Elimination factors of every (kx, ky) column's z system (or of the
-// transposed systems): two arrays of nz nx (ny/2+1) doubles; and the sweep.
-cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, double *th_g, const double *kx2,
-                                  const double *ky2, const double *cl, const double *cr, bool transposed,
-                                  cudaStream_t s);
-cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *th_g,
-                                  const double *cl, const double *cr, cudaStream_t s, bool transposed = false);
+// Inverse pivots of every (kx, ky) column's z system (or of the transposed
+// systems): nz nx (ny/2+1) doubles; and the sweep.
+cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, const double *kx2, const double *ky2,
+                                  const double *cl, const double *cr, bool transposed, cudaStream_t s);
+cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *cl,
+                                  const double *cr, cudaStream_t s, bool transposed = false);
 cudaError_t launch_project(const SlcParams &P, const double *phi_zmajor, TriMut f, double *p,
                            const double *dz_c, double dt, cudaStream_t s);
 // bulk: partial sums of u*dz_f over the interior (shift c added first when
@@ -184,7 +183,7 @@ struct EnsInst {
     double *mid[3];                 // U* = 2 V^n - V^{n-1}, ghost-shaped
     const double *dzf, *dzc, *kx2, *ky2, *cl, *cr;
     double *rhs, *hat;              // Poisson workspaces (inside a group's FFT pools)
-    const double *th_id, *th_g;     // Poisson elimination factors
+    const double *th_id;            // Poisson inverse pivots
     const double *zs_uv, *zs_w;     // z-solve tables at dt_eff = 2 dt / 3
     double *partials, *scal;        // kBulkBlocks partial sums; [shift, forcing]
     unsigned long long *ncl;        // departure-clamp counter
