@@ -30,6 +30,7 @@
 #include <cufft.h>
 
 #include <algorithm>
+#include <climits>
 #include <string>
 
 #include "slc_grid.h"
@@ -291,9 +292,14 @@ __device__ __forceinline__ void trace_forward(const SlcParams &P, const V3 &M, c
 // The records of the trilinear samples, per field c of U*: key = base node
 // (i0 * ny + j0) * NZ + k0, payload (tx, ty, wz1, coefficient).  Written where
 // the sample's stencils are at hand, one array per field, so that the
-// transposes sort and read nothing else.
+// transposes sort and read nothing else.  w's base node is u's and v's in part
+// (x of v, y of u, the face cell below or at their centre interval): k_w_keys
+// makes its keys from theirs when they are sorted, with the cell's half in the
+// top bit of u's.
+constexpr int kHalfBit = INT_MIN, kKeyMask = INT_MAX;
+
 struct TriOut {
-    int *key[3];
+    int *key[2];
     double4 *pay[3];
 };
 
@@ -303,10 +309,23 @@ __device__ __forceinline__ void write_records(const SlcParams &P, const TriShare
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const TriPiece q = tri_piece(P, c, t);
-        const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
-        out.key[c][r] = (q.i0 * P.ny + q.j0) * NZ + q.k0;
+        if (c < 2) {
+            const int key = (q.i0 * P.ny + q.j0) * (P.nz + 2) + q.k0;
+            out.key[c][r] = c == 0 && t.kc != t.kf ? key | kHalfBit : key;
+        }
         out.pay[c][r] = make_double4(q.tx, q.ty, q.wz1, coef[c]);
     }
+}
+
+__global__ void k_w_keys(SlcParams P, const int *__restrict__ ku, const int *__restrict__ kv, long long n,
+                         int *__restrict__ kw)
+{
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const int NZ = P.nz + 2;
+    const int u = ku[r] & kKeyMask, ib = kv[r] / (P.ny * NZ);
+    const int col = u / NZ, kc = u - col * NZ, jb = col % P.ny;
+    kw[r] = (ib * P.ny + jb) * (P.nz + 1) + kc - (ku[r] < 0 ? 1 : 0);
 }
 
 __device__ __forceinline__ void trace_backward(const SlcParams &P, const V3 &M, const FootTrace &T,
@@ -454,7 +473,7 @@ __global__ void k_izero(int *a, long long n)
 __global__ void k_count(const int *__restrict__ keys, long long n, int *counts)
 {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n) atomicAdd(counts + keys[r], 1);
+    if (r < n) atomicAdd(counts + (keys[r] & kKeyMask), 1);
 }
 
 constexpr int kScanT = 1024;
@@ -540,7 +559,7 @@ __global__ void k_place(const int *__restrict__ keys, long long n, const int *__
 {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
-    const int key = keys[r];
+    const int key = keys[r] & kKeyMask;
     const int pos = starts[key] + atomicAdd(fill + key, 1);
     order[pos] = (int)r;
 }
@@ -901,21 +920,28 @@ __global__ void k_axpy(double *y, const double *__restrict__ x, double a, long l
 
 // ---- host side -------------------------------------------------------------------
 
+// One allocation.  What the gathers' transposes use (near, far, keys, order, W,
+// kz, part) and what the trajectory records' use at the end (order, kw, part,
+// lam_mid) share a region, and within the former part shares near's and keys':
+// near and keys are read before part is written.  At order 6 and two iterations
+// 1.15 kB per cell.
 struct AdjWS {
-    long long n_c[3] = {0, 0, 0}, ntot = 0, nkeys_max = 0, nrec_max = 0;
-    double4 *rec_near = nullptr, *rec_far = nullptr;
+    long long n_c[3] = {0, 0, 0}, ntot = 0, nrec_max = 0;
     TriOut tri{};
-    int *keys = nullptr, *order = nullptr, *counts = nullptr, *starts = nullptr, *fill = nullptr;
-    int *sums = nullptr, *total = nullptr;
-    double *lam_mid[3] = {nullptr, nullptr, nullptr};
+    int *counts = nullptr, *starts = nullptr, *sums = nullptr, *total = nullptr;
     double *zs_tab = nullptr, zs_dt = 0.0;  // z-solve tables of the transposed systems, at zs_dt
-    double *th_id = nullptr;  // Poisson inverse pivots of the transposed systems
     double *partials = nullptr, *S = nullptr;
-    double *W = nullptr;  // sorted gather weights, 3 O arrays of n_c[0]
-    int *kz = nullptr;    // sorted gather records' first z node
-    // partial sums over the bases: 8 trilinear corners, or O x offsets of a
-    // gather's transpose (arrays of nkeys_max)
-    double *part = nullptr;
+    struct Gather {
+        double4 *near, *far;
+        int *keys, *order, *kz;  // kz: sorted gather records' first z node
+        double *W;               // sorted gather weights, 3 O arrays of n_c[0]
+        double *part;            // partial sums over the bases per x offset, O arrays
+    } ga{};
+    struct Tri {
+        int *order, *kw;
+        double *part;            // per corner, 8 arrays
+        double *lam_mid[3];
+    } tr{};
 };
 
 namespace {
@@ -929,82 +955,88 @@ namespace {
         }                                                                                      \
     } while (0)
 
-template <typename T>
-int adj_alloc(slc_grid *g, T **p, size_t n, const char *what)
-{
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, n * sizeof(T) > 0 ? n * sizeof(T) : 16);
-    if (e != cudaSuccess) {
-        g->err = std::string("cudaMalloc ") + what + ": " + cudaGetErrorString(e);
-        return SLC_E_NOMEM;
+// Hands out 256-byte aligned pieces of base, or only measures without one.
+struct Carve {
+    char *base;
+    size_t off = 0, top = 0;
+    template <typename T>
+    T *take(size_t n)
+    {
+        T *p = base ? (T *)(base + off) : nullptr;
+        off += (n * sizeof(T) + 255) & ~(size_t)255;
+        top = std::max(top, off);
+        return p;
     }
-    g->allocs.push_back(q);
-    *p = (T *)q;
-    return SLC_OK;
+};
+
+size_t adj_layout(const slc_grid *g, AdjWS *w, char *base)
+{
+    const SlcParams &P = g->P;
+    const size_t nkeys = (size_t)P.nx * P.ny * (P.nz + 2), nrec = (size_t)w->nrec_max, n0 = (size_t)w->n_c[0];
+    Carve c{base};
+    for (int q = 0; q < 2; ++q) w->tri.key[q] = c.take<int>(nrec);
+    for (int q = 0; q < 3; ++q) w->tri.pay[q] = c.take<double4>(nrec);
+    w->counts = c.take<int>(nkeys + 1);
+    w->starts = c.take<int>(nkeys + 1);
+    w->sums = c.take<int>((nkeys + 1 + kScanT - 1) / kScanT);
+    w->total = c.take<int>(1);
+    w->zs_tab = c.take<double>(zsolve_table_doubles(P.nz));
+    w->partials = c.take<double>(kSumBlocks);
+    w->S = c.take<double>(1);
+    const size_t shared = c.off;
+    w->ga.far = c.take<double4>(n0);
+    w->ga.order = c.take<int>(n0);
+    w->ga.kz = c.take<int>(n0);
+    w->ga.W = c.take<double>((size_t)3 * P.order * n0);
+    const size_t behind = c.off;
+    w->ga.near = c.take<double4>(n0);
+    w->ga.keys = c.take<int>(n0);
+    c.off = behind;
+    w->ga.part = c.take<double>((size_t)P.order * nkeys);
+    c.off = shared;
+    w->tr.order = c.take<int>(nrec);
+    w->tr.kw = c.take<int>(nrec);
+    w->tr.part = c.take<double>(8 * nkeys);
+    for (int q = 0; q < 3; ++q) w->tr.lam_mid[q] = c.take<double>(g->ghost_elems[q]);
+    return c.top;
 }
 
-int ensure_adj(slc_grid *g, cudaStream_t s)
+int ensure_adj(slc_grid *g)
 {
     if (g->adj) return SLC_OK;
     const SlcParams &P = g->P;
-    AdjWS *w = new AdjWS();
+    AdjWS w;
     const long long plane = (long long)P.nx * P.ny;
-    w->n_c[0] = w->n_c[1] = plane * P.nz;
-    w->n_c[2] = plane * (P.nz - 1);
-    w->ntot = w->n_c[0] + w->n_c[1] + w->n_c[2];
-    const long long slots = 2LL * P.n_iters - 1;
-    w->nkeys_max = plane * (P.nz + 2);
-    w->nrec_max = slots * w->ntot;
-    const long long nb = (w->nkeys_max + 1 + kScanT - 1) / kScanT;
-    int rc = adj_alloc(g, &w->rec_near, (size_t)w->n_c[0], "adjoint near records");
-    if (!rc) rc = adj_alloc(g, &w->rec_far, (size_t)w->n_c[0], "adjoint far records");
-    for (int c = 0; c < 3 && !rc; ++c) {
-        rc = adj_alloc(g, &w->tri.key[c], (size_t)w->nrec_max, "adjoint trajectory keys");
-        if (!rc) rc = adj_alloc(g, &w->tri.pay[c], (size_t)w->nrec_max, "adjoint trajectory records");
-    }
-    if (!rc) rc = adj_alloc(g, &w->keys, (size_t)w->n_c[0], "adjoint keys");
-    if (!rc) rc = adj_alloc(g, &w->order, (size_t)w->nrec_max, "adjoint order");
-    if (!rc) rc = adj_alloc(g, &w->counts, (size_t)w->nkeys_max + 1, "adjoint counts");
-    if (!rc) rc = adj_alloc(g, &w->starts, (size_t)w->nkeys_max + 1, "adjoint starts");
-    if (!rc) rc = adj_alloc(g, &w->fill, (size_t)w->nkeys_max + 1, "adjoint fill");
-    if (!rc) rc = adj_alloc(g, &w->sums, (size_t)nb, "adjoint scan sums");
-    if (!rc) rc = adj_alloc(g, &w->total, (size_t)1, "adjoint scan total");
-    for (int c = 0; c < 3 && !rc; ++c) rc = adj_alloc(g, &w->lam_mid[c], g->ghost_elems[c], "adjoint U*");
-    if (!rc) rc = adj_alloc(g, &w->zs_tab, zsolve_table_doubles(P.nz), "adjoint z-solve tables");
-    if (!rc) rc = adj_alloc(g, &w->partials, (size_t)kSumBlocks, "adjoint partials");
-    if (!rc) rc = adj_alloc(g, &w->S, (size_t)1, "adjoint sum");
-    if (!rc) rc = adj_alloc(g, &w->W, (size_t)3 * SLC_MAX_ORDER * w->n_c[0], "adjoint gather weights");
-    if (!rc) rc = adj_alloc(g, &w->kz, (size_t)w->n_c[0], "adjoint gather z bases");
-    if (!rc) rc = adj_alloc(g, &w->part, (size_t)8 * w->nkeys_max, "adjoint partial sums");
-    const size_t ncplx = (size_t)P.nz * P.nx * (P.ny / 2 + 1);
-    if (!rc) rc = adj_alloc(g, &w->th_id, ncplx, "adjoint Poisson inverse pivots");
-    if (rc) {
-        delete w;
-        return rc;
-    }
-    cudaError_t e = launch_thomas_factors(P, w->th_id, g->kx2, g->ky2, g->cl, g->cr, true, s);
+    w.n_c[0] = w.n_c[1] = plane * P.nz;
+    w.n_c[2] = plane * (P.nz - 1);
+    w.ntot = w.n_c[0] + w.n_c[1] + w.n_c[2];
+    w.nrec_max = (2LL * P.n_iters - 1) * w.ntot;
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, adj_layout(g, &w, nullptr));
     if (e != cudaSuccess) {
-        delete w;
-        g->err = std::string("adjoint Poisson inverse pivots: ") + cudaGetErrorString(e);
-        return SLC_E_CUDA;
+        cudaGetLastError();  // reported here
+        g->err = std::string("cudaMalloc adjoint workspace: ") + cudaGetErrorString(e);
+        return SLC_E_NOMEM;
     }
-    g->adj = w;
+    g->allocs.push_back(p);
+    adj_layout(g, &w, (char *)p);
+    g->adj = new AdjWS(w);
     return SLC_OK;
 }
 
-// Counting sort of keys[0, n) over nkeys keys into w->order / w->starts.
-int sort_records(slc_grid *g, AdjWS *w, const int *keys, long long n, long long nkeys, cudaStream_t s)
+// Counting sort of keys[0, n) over nkeys keys into order / w->starts.
+int sort_records(slc_grid *g, AdjWS *w, const int *keys, long long n, long long nkeys, int *order, cudaStream_t s)
 {
     k_izero<<<nblk(nkeys + 1), kT, 0, s>>>(w->counts, nkeys + 1);
-    k_izero<<<nblk(nkeys + 1), kT, 0, s>>>(w->fill, nkeys + 1);
     if (n > 0) k_count<<<nblk(n), kT, 0, s>>>(keys, n, w->counts);
     const long long m = nkeys + 1;
     const int nb = (int)((m + kScanT - 1) / kScanT);
     k_scan_blocks<<<nb, kScanT, 0, s>>>(w->counts, w->starts, w->sums, m);
     k_scan_sums<<<1, kScanT, 0, s>>>(w->sums, nb, w->total);
     k_scan_add<<<nb, kScanT, 0, s>>>(w->starts, w->sums, m);
-    if (n > 0) k_place<<<nblk(n), kT, 0, s>>>(keys, n, w->starts, w->fill, w->order);
-    k_sort_segments<<<nblk(nkeys), kT, 0, s>>>(w->starts, nkeys, w->order);
+    k_izero<<<nblk(nkeys + 1), kT, 0, s>>>(w->counts, nkeys + 1);  // now each key's records placed
+    if (n > 0) k_place<<<nblk(n), kT, 0, s>>>(keys, n, w->starts, w->counts, order);
+    k_sort_segments<<<nblk(nkeys), kT, 0, s>>>(w->starts, nkeys, order);
     count_launches(n > 0 ? 9 : 7);
     ADJ_CK(cudaGetLastError(), "adjoint record sort");
     return SLC_OK;
@@ -1041,13 +1073,13 @@ int sl_adjoint_t(slc_grid *g, AdjWS *w, const V3 &M, const double *const cur[3],
         // points -> records
         if (C == 0)
             k_sl_adj_points<0, O, MODE><<<nblk(n), kT, 0, s>>>(P, M, cur[0], fnm1[0], lam_hat[0], dt,
-                                                               w->rec_near, w->rec_far, w->tri, pbase[0], w->ntot);
+                                                               w->ga.near, w->ga.far, w->tri, pbase[0], w->ntot);
         else if (C == 1)
             k_sl_adj_points<1, O, MODE><<<nblk(n), kT, 0, s>>>(P, M, cur[1], fnm1[1], lam_hat[1], dt,
-                                                               w->rec_near, w->rec_far, w->tri, pbase[1], w->ntot);
+                                                               w->ga.near, w->ga.far, w->tri, pbase[1], w->ntot);
         else
             k_sl_adj_points<2, O, MODE><<<nblk(n), kT, 0, s>>>(P, M, cur[2], fnm1[2], lam_hat[2], dt,
-                                                               w->rec_near, w->rec_far, w->tri, pbase[2], w->ntot);
+                                                               w->ga.near, w->ga.far, w->tri, pbase[2], w->ntot);
         count_launches(1);
         const int NZ = C < 2 ? P.nz + 2 : P.nz + 1;
         const long long nkeys = (long long)P.nx * P.ny * NZ;
@@ -1056,26 +1088,26 @@ int sl_adjoint_t(slc_grid *g, AdjWS *w, const V3 &M, const double *const cur[3],
         const long long ncols = (long long)P.nx * nseg * NZ;
         // near foot -> lam_cur[C]; far foot -> lam_prev[C]
         for (int foot = 0; foot < (MODE == 2 ? 2 : 1); ++foot) {
-            const double4 *rec = foot == 0 ? w->rec_near : w->rec_far;
+            const double4 *rec = foot == 0 ? w->ga.near : w->ga.far;
             double *dst = foot == 0 ? lam_cur[C] : lam_prev[C];
-            if (C == 0) k_gather_keys<0, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->keys);
-            else if (C == 1) k_gather_keys<1, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->keys);
-            else k_gather_keys<2, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->keys);
+            if (C == 0) k_gather_keys<0, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->ga.keys);
+            else if (C == 1) k_gather_keys<1, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->ga.keys);
+            else k_gather_keys<2, O><<<nblk(n), kT, 0, s>>>(P, rec, n, w->ga.keys);
             count_launches(1);
-            int rc = sort_records(g, w, w->keys, n, nkeys, s);
+            int rc = sort_records(g, w, w->ga.keys, n, nkeys, w->ga.order, s);
             if (rc) return rc;
             if (C == 0) {
-                k_sorted_weights<0, O><<<nblk(n), kT, 0, s>>>(P, rec, w->order, n, w->W, w->kz);
-                k_pull_columns<0, O><<<nblk(ncols), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, nseg, seg_len, w->part);
-                k_pull_rows<0, O><<<nblk(nkeys), kT, 0, s>>>(P, w->part, dst);
+                k_sorted_weights<0, O><<<nblk(n), kT, 0, s>>>(P, rec, w->ga.order, n, w->ga.W, w->ga.kz);
+                k_pull_columns<0, O><<<nblk(ncols), kT, 0, s>>>(P, w->ga.W, w->ga.kz, n, w->starts, nseg, seg_len, w->ga.part);
+                k_pull_rows<0, O><<<nblk(nkeys), kT, 0, s>>>(P, w->ga.part, dst);
             } else if (C == 1) {
-                k_sorted_weights<1, O><<<nblk(n), kT, 0, s>>>(P, rec, w->order, n, w->W, w->kz);
-                k_pull_columns<1, O><<<nblk(ncols), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, nseg, seg_len, w->part);
-                k_pull_rows<1, O><<<nblk(nkeys), kT, 0, s>>>(P, w->part, dst);
+                k_sorted_weights<1, O><<<nblk(n), kT, 0, s>>>(P, rec, w->ga.order, n, w->ga.W, w->ga.kz);
+                k_pull_columns<1, O><<<nblk(ncols), kT, 0, s>>>(P, w->ga.W, w->ga.kz, n, w->starts, nseg, seg_len, w->ga.part);
+                k_pull_rows<1, O><<<nblk(nkeys), kT, 0, s>>>(P, w->ga.part, dst);
             } else {
-                k_sorted_weights<2, O><<<nblk(n), kT, 0, s>>>(P, rec, w->order, n, w->W, w->kz);
-                k_pull_columns<2, O><<<nblk(ncols), kT, 0, s>>>(P, w->W, w->kz, n, w->starts, nseg, seg_len, w->part);
-                k_pull_rows<2, O><<<nblk(nkeys), kT, 0, s>>>(P, w->part, dst);
+                k_sorted_weights<2, O><<<nblk(n), kT, 0, s>>>(P, rec, w->ga.order, n, w->ga.W, w->ga.kz);
+                k_pull_columns<2, O><<<nblk(ncols), kT, 0, s>>>(P, w->ga.W, w->ga.kz, n, w->starts, nseg, seg_len, w->ga.part);
+                k_pull_rows<2, O><<<nblk(nkeys), kT, 0, s>>>(P, w->ga.part, dst);
             }
             count_launches(3);
         }
@@ -1091,18 +1123,23 @@ int sl_adjoint_t(slc_grid *g, AdjWS *w, const V3 &M, const double *const cur[3],
     // trajectory records -> lam_U* per field
     const long long nrec = (long long)(MODE == 2 ? 2 * P.n_iters - 1 : P.n_iters) * w->ntot;
     for (int c = 0; c < 3; ++c) {
-        ADJ_CK(cudaMemsetAsync(w->lam_mid[c], 0, g->ghost_elems[c] * sizeof(double), s), "memset");
+        ADJ_CK(cudaMemsetAsync(w->tr.lam_mid[c], 0, g->ghost_elems[c] * sizeof(double), s), "memset");
         const int NZ = c < 2 ? P.nz + 2 : P.nz + 1;
         const long long nkeys = (long long)P.nx * P.ny * NZ;
-        int rc = sort_records(g, w, w->tri.key[c], nrec, nkeys, s);
+        const int *keys = c < 2 ? w->tri.key[c] : w->tr.kw;
+        if (c == 2) {
+            k_w_keys<<<nblk(nrec), kT, 0, s>>>(P, w->tri.key[0], w->tri.key[1], nrec, w->tr.kw);
+            count_launches(1);
+        }
+        int rc = sort_records(g, w, keys, nrec, nkeys, w->tr.order, s);
         if (rc) return rc;
-        k_tri_segsum<<<nblk(nkeys), kT, 0, s>>>(w->tri.pay[c], w->order, w->starts, nkeys, w->part);
-        k_pull_tri<<<nblk(nkeys), kT, 0, s>>>(P, c, w->part, w->lam_mid[c]);
+        k_tri_segsum<<<nblk(nkeys), kT, 0, s>>>(w->tri.pay[c], w->tr.order, w->starts, nkeys, w->tr.part);
+        k_pull_tri<<<nblk(nkeys), kT, 0, s>>>(P, c, w->tr.part, w->tr.lam_mid[c]);
         count_launches(2);
         // U* = 2 V^n - V^{n-1} (BDF2) or V^n (BDF1)
         const long long ne = (long long)g->ghost_elems[c];
-        k_axpy<<<148 * 8, kT, 0, s>>>(lam_cur[c], w->lam_mid[c], MODE == 2 ? 2.0 : 1.0, ne);
-        if (MODE == 2) k_axpy<<<148 * 8, kT, 0, s>>>(lam_prev[c], w->lam_mid[c], -1.0, ne);
+        k_axpy<<<148 * 8, kT, 0, s>>>(lam_cur[c], w->tr.lam_mid[c], MODE == 2 ? 2.0 : 1.0, ne);
+        if (MODE == 2) k_axpy<<<148 * 8, kT, 0, s>>>(lam_prev[c], w->tr.lam_mid[c], -1.0, ne);
         count_launches(MODE == 2 ? 2 : 1);
     }
     ADJ_CK(cudaGetLastError(), "SL adjoint");
@@ -1182,7 +1219,8 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
     }
     cudaSetDevice(g->device);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = ensure_adj(g, s);
+    int rc = ensure_adj(g);
+    if (!rc) rc = slc_grid_ensure_pivots(g, s);
     if (rc) return rc;
     AdjWS *w = g->adj;
     const SlcParams &P = g->P;
@@ -1206,7 +1244,7 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
         g->err = "cufftExecD2Z (adjoint)";
         return SLC_E_CUFFT;
     }
-    ADJ_CK(launch_thomas_poisson(P, g->hat, w->th_id, g->cl, g->cr, s, true), "Poisson Thomas adjoint");
+    ADJ_CK(launch_thomas_poisson(P, g->hat, g->th_id, g->cl, g->cr, s, true), "Poisson Thomas adjoint");
     if (cufftSetStream(g->inv, s) != CUFFT_SUCCESS ||
         cufftExecZ2D(g->inv, (cufftDoubleComplex *)g->hat, g->rhs) != CUFFT_SUCCESS) {
         g->err = "cufftExecZ2D (adjoint)";

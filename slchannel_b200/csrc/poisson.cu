@@ -184,17 +184,16 @@ struct Row3 {
     double a, b, c;
 };
 
-template <bool T>
 __device__ __forceinline__ Row3 poisson_row(const double *__restrict__ cl, const double *__restrict__ cr, double k2,
                                             int nz, int k, bool pinned)
 {
     Row3 r;
-    r.a = poisson_down<T>(cl, cr, k, pinned);
+    r.a = poisson_down<false>(cl, cr, k, pinned);
     r.b = -(cl[k] + cr[k] + k2);
     if (k == 0) r.b += cl[0];
     if (k == nz - 1) r.b += cr[nz - 1];
     if (pinned && k == 0) r.b = 1.0;
-    r.c = poisson_up<T>(cl, cr, nz, k, pinned);
+    r.c = poisson_up<false>(cl, cr, nz, k, pinned);
     return r;
 }
 
@@ -205,14 +204,14 @@ __device__ __forceinline__ Row3 poisson_row(const double *__restrict__ cl, const
 // grid alone: k_thomas_factors computes them once per handle, at its first
 // projection (row k of column col at k * ncol + col, the meeting row's included).
 // A row's pivot ratio is its outward coupling times its inverse pivot, so the one
-// table serves both halves of a sweep.  A sweep then has two dependent operations
+// table serves both halves of a sweep; and the transposed systems' too, whose
+// pivots b_k - a_k c_{k-1} / p_{k-1} are the same.  A sweep then has two dependent operations
 // per row where dividing by the pivot on the way was a chain of some thirty:
 // 12.2 -> 6.3 us at 32^3, 24 -> 12 us at 64^3, 211 -> 109 us at 256^3 (0.7 GB: bound
 // there by the traffic, which the table leaves as it was: one word read where a
 // pivot ratio was stored).  The table alone, with the loads of a row still tested
 // one by one behind the chain, was no faster at 64^3 (29 us): the batches below
 // matter as much.
-template <bool T>
 __global__ void __launch_bounds__(256) k_thomas_factors(SlcParams P, double *__restrict__ th_id,
                                                         const double *__restrict__ kx2,
                                                         const double *__restrict__ ky2,
@@ -229,18 +228,18 @@ __global__ void __launch_bounds__(256) k_thomas_factors(SlcParams P, double *__r
     const bool pinned = col == 0;
     double gt = 0.0, gb = 0.0;
     for (int k = 0; k < m; ++k) {
-        const Row3 R = poisson_row<T>(cl, cr, k2, nz, k, pinned);
+        const Row3 R = poisson_row(cl, cr, k2, nz, k, pinned);
         const double id = 1.0 / (R.b - R.a * gt);
         gt = R.c * id;
         th_id[(size_t)k * ncol + col] = id;
     }
     for (int k = nz - 1; k > m; --k) {
-        const Row3 R = poisson_row<T>(cl, cr, k2, nz, k, pinned);
+        const Row3 R = poisson_row(cl, cr, k2, nz, k, pinned);
         const double id = 1.0 / (R.b - R.c * gb);
         gb = R.a * id;
         th_id[(size_t)k * ncol + col] = id;
     }
-    const Row3 R = poisson_row<T>(cl, cr, k2, nz, m, pinned);
+    const Row3 R = poisson_row(cl, cr, k2, nz, m, pinned);
     th_id[(size_t)m * ncol + col] = 1.0 / (R.b - R.a * gt - R.c * gb);
 }
 
@@ -711,12 +710,10 @@ cudaError_t launch_divergence(const SlcParams &P, Tri f, const double *dz_f, dou
 }
 
 cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, const double *kx2, const double *ky2,
-                                  const double *cl, const double *cr, bool transposed,
-                                  cudaStream_t s)
+                                  const double *cl, const double *cr, cudaStream_t s)
 {
     const unsigned nb = (unsigned)(((long long)P.nx * (P.ny / 2 + 1) + 255) / 256);
-    if (transposed) k_thomas_factors<true><<<nb, 256, 0, s>>>(P, th_id, kx2, ky2, cl, cr);
-    else k_thomas_factors<false><<<nb, 256, 0, s>>>(P, th_id, kx2, ky2, cl, cr);
+    k_thomas_factors<<<nb, 256, 0, s>>>(P, th_id, kx2, ky2, cl, cr);
     count_launches(1);
     return cudaGetLastError();
 }

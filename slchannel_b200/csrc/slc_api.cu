@@ -158,7 +158,7 @@ bool capturing(cudaStream_t s);
 int ensure_pivots(slc_grid *g, cudaStream_t s)
 {
     if (g->th_valid) return SLC_OK;
-    SLC_CK(launch_thomas_factors(g->P, g->th_id, g->kx2, g->ky2, g->cl, g->cr, false, s), "Poisson inverse pivots");
+    SLC_CK(launch_thomas_factors(g->P, g->th_id, g->kx2, g->ky2, g->cl, g->cr, s), "Poisson inverse pivots");
     g->th_valid = !capturing(s);
     return SLC_OK;
 }

@@ -111,10 +111,10 @@ cudaError_t launch_div_pack(const SlcParams &P, Tri f, const double *dz_f, doubl
                             double *rhs_zmajor, cudaStream_t s);
 cudaError_t launch_divergence(const SlcParams &P, Tri f, const double *dz_f, double *div,
                               cudaStream_t s);
-// Inverse pivots of every (kx, ky) column's z system (or of the transposed
-// systems): nz nx (ny/2+1) doubles; and the sweep.
+// Inverse pivots of every (kx, ky) column's z system (and of the transposed
+// system): nz nx (ny/2+1) doubles; and the sweep.
 cudaError_t launch_thomas_factors(const SlcParams &P, double *th_id, const double *kx2, const double *ky2,
-                                  const double *cl, const double *cr, bool transposed, cudaStream_t s);
+                                  const double *cl, const double *cr, cudaStream_t s);
 cudaError_t launch_thomas_poisson(const SlcParams &P, double *hat, const double *th_id, const double *cl,
                                   const double *cr, cudaStream_t s, bool transposed = false);
 cudaError_t launch_project(const SlcParams &P, const double *phi_zmajor, TriMut f, double *p,

@@ -133,3 +133,35 @@ def test_adjoint_refuses_unsupported_forms(attr, value):
     V0 = tuple(t.clone() for t in (f.u, f.v, f.w))
     with pytest.raises(ValueError, match="noninc"):
         A.loss_of(f, V0, dt, 1, A.smooth_mask(f, seed=1))
+
+
+def _first_adjoint_bytes(nx, ny, nz, order):
+    flow = _flow(nx, ny, nz, 2 * math.pi, math.pi, 2800.0, 0.02, order)
+    V = [torch.rand_like(t) for t in (flow.u, flow.v, flow.w)]
+    flow.set_state(*V)
+    for _ in range(2):
+        flow.step_sl_bdf2(0.02)  # the step's own workspaces
+    st = A._Stepper(flow)
+    lams = [tuple(torch.rand_like(t) for t in V) for _ in range(3)]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    st.adjoint(1, (flow.u_nm1, flow.v_nm1, flow.w_nm1), (flow.u, flow.v, flow.w), *lams, 0.02)
+    torch.cuda.synchronize()
+    return free - torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("order", [6, 4])
+def test_adjoint_workspace_size(order):
+    """The workspace stays within what it took with one 48-byte record per
+    trajectory sample, unpacked per field (84 bytes a sample and its place in the
+    sort, 8 weight slots per order, separate sums and sweeps), up to the
+    allocator's 2 MB granules."""
+    nx, ny, nz = 96, 80, 64
+    _first_adjoint_bytes(12, 10, 16, order)  # loads the kernels
+    n, nodes = nx * ny * nz, nx * ny * (nz + 2)
+    samples = 3 * (3 * n - nx * ny)
+    ghosts = (nx + 2) * (ny + 2) * (nz + 2)
+    most = samples * (48 + 32 + 4 + 4) + n * (2 * 32 + 3 * 8 * 8 + 4 + 3 * 8) + nodes * (8 * 8 + 3 * 4) + 3 * 8 * ghosts
+    used = _first_adjoint_bytes(nx, ny, nz, order)
+    print(f"order {order}: {used / n:.0f} bytes a cell, at most {most / n:.0f}")
+    assert 0 < used <= most + (4 << 20)
