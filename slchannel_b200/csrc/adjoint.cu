@@ -929,7 +929,8 @@ struct AdjWS {
     long long n_c[3] = {0, 0, 0}, ntot = 0, nrec_max = 0;
     TriOut tri{};
     int *counts = nullptr, *starts = nullptr, *sums = nullptr, *total = nullptr;
-    double *zs_tab = nullptr, zs_dt = 0.0;  // z-solve tables of the transposed systems, at zs_dt
+    // z-solve tables of the transposed systems: at zs_dt, and those of graphs
+    double *zs_tab = nullptr, zs_dt = 0.0;
     double *partials = nullptr, *S = nullptr;
     struct Gather {
         double4 *near, *far;
@@ -980,7 +981,7 @@ size_t adj_layout(const slc_grid *g, AdjWS *w, char *base)
     w->starts = c.take<int>(nkeys + 1);
     w->sums = c.take<int>((nkeys + 1 + kScanT - 1) / kScanT);
     w->total = c.take<int>(1);
-    w->zs_tab = c.take<double>(zsolve_table_doubles(P.nz));
+    w->zs_tab = c.take<double>(2 * zsolve_table_doubles(P.nz));
     w->partials = c.take<double>(kSumBlocks);
     w->S = c.take<double>(1);
     const size_t shared = c.off;
@@ -1253,13 +1254,18 @@ int slc_adjoint_step(slc_grid *g, int mode, double *const cur[3], double *const 
     k_divT<<<nblk(n), kT, 0, s>>>(P, g->rhs, g->dzf, 1.0, lam_next[0], lam_next[1], lam_next[2]);
     count_launches(1);
     // 3. z-solve: A^T x = d per column, the forward's kernel with the tables of
-    // the transposed systems
-    double *tab_w = w->zs_tab + zsolve_table_doubles(P.nz) / 2;
-    if (w->zs_dt != dt_eff) {
-        ADJ_CK(launch_zsolve_tables(P, g->dzc, g->dzf, dt_eff, w->zs_tab, tab_w, s, true), "z-solve adjoint tables");
-        w->zs_dt = dt_eff;
+    // the transposed systems; a graph's launch fills its own tables each time it
+    // runs, since it runs after calls at other dt
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    ADJ_CK(cudaStreamIsCapturing(s, &cap), "capture status");
+    const bool eager = cap == cudaStreamCaptureStatusNone;
+    double *tab = w->zs_tab + (eager ? 0 : zsolve_table_doubles(P.nz));
+    double *tab_w = tab + zsolve_table_doubles(P.nz) / 2;
+    if (!eager || w->zs_dt != dt_eff) {
+        ADJ_CK(launch_zsolve_tables(P, g->dzc, g->dzf, dt_eff, tab, tab_w, s, true), "z-solve adjoint tables");
+        if (eager) w->zs_dt = dt_eff;
     }
-    ADJ_CK(launch_zsolve(P, TriMut{lam_next[0], lam_next[1], lam_next[2]}, w->zs_tab, tab_w, s), "z-solve adjoint");
+    ADJ_CK(launch_zsolve(P, TriMut{lam_next[0], lam_next[1], lam_next[2]}, tab, tab_w, s), "z-solve adjoint");
     ADJ_CK(cudaGetLastError(), "projection / z-solve adjoint");
     // 4. SL predictor: U* recomputed
     V3 M;

@@ -165,3 +165,48 @@ def test_adjoint_workspace_size(order):
     used = _first_adjoint_bytes(nx, ny, nz, order)
     print(f"order {order}: {used / n:.0f} bytes a cell, at most {most / n:.0f}")
     assert 0 < used <= most + (4 << 20)
+
+
+def test_adjoint_in_a_graph_beside_other_time_steps():
+    """A captured adjoint step keeps its own dt whatever runs between capture and
+    replay, and leaves the tables of calls at other dt alone."""
+    dt1, dt2 = 0.02, 0.05
+    flow = _flow(14, 12, 18, 2 * math.pi, math.pi, 200.0, dt1, 4)
+    g = torch.Generator().manual_seed(5)
+    rand = lambda t: torch.randn(t.shape, generator=g, dtype=torch.float64).to(t.device)  # noqa: E731
+    flow.set_state(*(rand(t) for t in (flow.u, flow.v, flow.w)))
+    for _ in range(2):
+        flow.step_sl_bdf2(dt1)
+    st = A._Stepper(flow)
+    cur, prev = (flow.u, flow.v, flow.w), (flow.u_nm1, flow.v_nm1, flow.w_nm1)
+    seeds = [rand(t) for t in cur]
+    lams = [tuple(torch.zeros_like(t) for t in cur) for _ in range(3)]
+
+    def run(dt):
+        for a, b in zip(lams[0], seeds):
+            a.copy_(b)
+        for t in (*lams[1], *lams[2]):
+            t.zero_()
+        st.adjoint(1, prev, cur, *lams, dt)
+
+    def result():
+        torch.cuda.synchronize()
+        return [t.clone() for lam in lams[1:] for t in lam]
+
+    run(dt2)
+    want2 = result()
+    run(dt1)
+    want1 = result()
+    assert not torch.equal(want1[0], want2[0])
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+        run(dt2)
+    torch.cuda.synchronize()
+    run(dt2)  # before the graph has run
+    assert all(torch.equal(a, b) for a, b in zip(result(), want2))
+    for _ in range(2):
+        run(dt1)
+        assert all(torch.equal(a, b) for a, b in zip(result(), want1))
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(result(), want2))
