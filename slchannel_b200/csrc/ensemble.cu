@@ -560,14 +560,12 @@ int slc_ensemble_bind(slc_ensemble *e, double *const *lev, double *const *p, con
             const SlcParams &P = e->grids[i]->P;
             const long long blocks = staged_blocks(P, e->mixed);
             if (blocks < SLC_ENS_STAGED_MIN_BLOCKS) continue;
-            if (!e->mixed && !tma_pays(P, ens_boxes(e->host_inst[i]))) {
-                e->staged[i] = 1;  // k_sl
-                continue;
-            }
+            e->staged[i] = !e->mixed;
+            if (!e->mixed && !tma_pays(P, ens_boxes(e->host_inst[i]))) continue;  // k_sl
             bool ready = false;
             int rs = slc_grid_ensure_staged(e->grids[i], &ready);
             if (rs) return efail(e, rs, std::string("instance ") + std::to_string(i) + ": " + e->grids[i]->err);
-            e->staged[i] = ready ? 1 : 0;
+            if (ready) e->staged[i] = 1;  // an FP64 one that is not runs k_sl
         }
     ENS_CK(cudaDeviceSynchronize(), "tables and memsets");
     int rc = upload_tables(e);

@@ -212,11 +212,12 @@ int ensure_mid(slc_grid *g)
 }
 
 // Padded node copies and tensor maps of the TMA-staged BDF2 gather; state -1
-// (L1 gather) when the grid is too shallow for a box or the driver lacks the
-// tensor-map entry point.
-int ensure_tma(slc_grid *g)
+// (k_sl) when the grid is too shallow for a box or the driver lacks the
+// tensor-map entry point, -2 when memory did not suffice for a caller that can
+// do without.
+int ensure_tma(slc_grid *g, bool optional)
 {
-    if (g->tma_state) return SLC_OK;
+    if (g->tma_state == 1 || g->tma_state == -1 || (g->tma_state == -2 && optional)) return SLC_OK;
     if (!tma_supported(g->P)) {
         g->tma_state = -1;
         return SLC_OK;
@@ -225,6 +226,10 @@ int ensure_tma(slc_grid *g)
     for (int q = 0; q < 6; ++q) off[q + 1] = off[q] + ((tma_padded_elems(g->P, q % 3) + 15) & ~(size_t)15);
     double *p = nullptr;
     int rc = dalloc(g, &p, off[6], "padded node copies");
+    if (rc && optional && cudaGetLastError() == cudaErrorMemoryAllocation) {
+        g->tma_state = -2;
+        return SLC_OK;
+    }
     if (rc) return rc;
     for (int q = 0; q < 6; ++q) g->tma.pad[q] = p + off[q];
     SLC_CK(tma_encode(g->P, g->tma), "tensor map encode");
@@ -301,7 +306,7 @@ int slc_grid_ensure_staged(slc_grid *g, bool *ready)
         if (!rc) *ready = g->tmx_state == 1;
     } else {
         rc = ensure_mid(g);
-        if (!rc) rc = ensure_tma(g);
+        if (!rc) rc = ensure_tma(g, true);
         if (!rc) *ready = g->tma_state == 1;
     }
     return rc;
@@ -478,9 +483,10 @@ int do_trace_gather_bdf2(slc_grid *g, const double *const cur[3], const double *
     // (choose_staged), else through L1 or with k_sl; order 4 keeps k_sl (64 loads
     // per foot leave too little to save).
     const bool forced = mode == kGatherStaged;
-    const bool copies = forced || (mode == kGatherDefault && g->P.order == 6 && tma_pays(g->P, true));
+    const bool copies = forced || (mode == kGatherDefault && g->P.order == 6 && tma_pays(g->P, true) &&
+                                   (g->tma_state || !capturing(s)));  // no allocation under capture
     int rc = ensure_mid(g);
-    if (!rc && copies) rc = ensure_tma(g);
+    if (!rc && copies) rc = ensure_tma(g, !forced);
     if (rc) return rc;
     const bool ready = copies && g->tma_state == 1;
     const bool staged = ready && (forced || choose_staged(g, s));

@@ -55,9 +55,9 @@ struct slc_grid {
     HostStep *host = nullptr;
     StatsWS *stats = nullptr;
     TmaSL tma{};
-    int tma_state = 0;        // 0 not tried, 1 ready, -1 unavailable (L1 gather path)
+    int tma_state = 0;        // 0 not tried, 1 ready, -1 unavailable, -2 out of memory (k_sl)
     TmaMixed tmx{};           // the mixed form's staged gather (padded FP32 copies, tensor maps)
-    int tmx_state = 0;        // as tma_state
+    int tmx_state = 0;        // 0 not tried, 1 ready, -1 unavailable (L1 gather)
     unsigned long long *dev_flags = nullptr;  // staged-gather statistics (launch_sl_tma)
     GatherChoice gchoice;
     size_t ghost_elems[4] = {0, 0, 0, 0};

@@ -130,3 +130,29 @@ def test_ensemble_leaves_the_boxes_for_fast_mean_flow_either_way(direction):
         torch.cuda.synchronize()
         handle = ctypes.c_void_p(N.lib().slc_ensemble_grid(ens._h, 0))
         assert (_blocks(handle) > 0) == boxes
+
+
+def test_step_without_memory_for_the_copies():
+    """Where the padded copies do not fit, the step runs k_sl instead of failing."""
+    n3, dt = (96, 64, 40), 0.01
+    fits, starved = _flow(n3, dt), _flow(n3, dt)
+    fits.step_sl_bdf2(dt)  # boxes
+    for f in (fits, starved):  # U* and the kernels
+        out = [torch.zeros_like(t) for t in (f.u, f.v, f.w)]
+        if f.u_nm1 is not None:
+            f._grid.call("slc_trace_gather_bdf2", *[N.ptr(t) for t in (f.u, f.v, f.w, f.u_nm1, f.v_nm1, f.w_nm1)],
+                         dt, *[N.ptr(t) for t in out], None, N.stream_of(f.u))
+    starved._next = starved._alloc_next()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    copies = 6 * 8 * (96 + 48) * (64 + 10) * 40
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - copies // 2, dtype=torch.uint8, device="cuda")
+    try:
+        starved.step_sl_bdf2(dt)
+        torch.cuda.synchronize()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert _blocks(starved._grid.handle) == 0 and _blocks(fits._grid.handle) > 0
+    for a, b in zip((fits.u, fits.v, fits.w, fits.p), (starved.u, starved.v, starved.w, starved.p)):
+        assert torch.equal(a, b)
