@@ -206,7 +206,7 @@ __device__ __forceinline__ bool box_fits(const int *r, int i0, int j0, const Slc
 // VN, VM: the padded copies of V^n and V^{n-1}.  TO, NI: trajectory order and
 // iterations, 0 to read them from P.  Tricubic trajectories take two blocks' 128
 // registers (step at 96x96x96: 1.42 ms at two blocks, 1.47 at three, 1.50 at four;
-// 1.63 with k_sl).
+// 1.47 with k_sl).
 template <int C, int O, int TO, int NI>
 __global__ void __launch_bounds__(kThreads, TO == 4 ? 2 : Box<O>::min_blocks)
     k_sl_tma(const __grid_constant__ SlcParams P, const __grid_constant__ Vel3X M, const __grid_constant__ NodeViewX VN,
@@ -466,25 +466,22 @@ bool tma_supported(const SlcParams &P)
 //   So three quarters of the lanes, from nx = 32.  A launch of less than one
 //   wave hardly feels idle lanes (24x16x48 1.08, and 0.66 of what it took from
 //   boxes with z along the lanes): there from nx = 24.
-// - Through L1, k_sl's lanes spread with the profile over 32 levels, all of
-//   it at nz = 32: 0.83 on 64x64x32, 0.85 on 128x96x64, 0.92 on 96x96x96, but 1.09
-//   on 64x128x128, 1.31 on 97x128x128, 1.02 on 120x120x120, 0.97 on 128x128x128.
-//   Up to 32 levels fewer lanes do (64x32 in y and z): from boxes 0.88 at nx 44,
-//   0.95 at 65, 1.04 at 33; through L1 0.87 at 48, 0.90 at 72, 0.97 at 44, 1.04 at 65.
-// - Tricubic trajectories read 64 nodes per sample through L1, so the same line
-//   as without boxes: 0.88 on 96x96x96, 0.84 on 192x128x96, 0.72 on 192x96x32, 0.97
-//   on 256x192x192, but 1.04 on 80x64x96, 1.03 on 97x75x81, 1.02 on 64x128x128; two
-//   iterations (unrolled, else 1.09 on 128x128x128).
+// - Through L1, k_sl's lanes spread with the profile over 32 levels, a whole
+//   channel at nz = 32: 0.88 on 64x64x32, 0.85 on 128x96x64, 0.96 on 96x96x96, but
+//   1.04 on 52x64x32, 1.09 on 64x128x128, 1.31 on 97x128x128, 1.02 on 120x120x120,
+//   0.97 on 128x128x128.
+// - Tricubic trajectories read 64 nodes per sample through L1, so the same line:
+//   0.91 on 64x64x32, 0.79 on 160x64x48, 0.97 on 96x96x96, 0.96 on 256x192x192, but
+//   1.05 on 80x64x32, 1.17 on 48x64x32; two iterations (unrolled, else 1.09 on 128x128x128).
 bool tma_pays(const SlcParams &P, bool staged)
 {
     const int tiles = (P.nx + kTI - 1) / kTI;
     const double lanes = (double)P.nx / (kTI * tiles);
-    const bool shallow = P.nz <= 32, cubic = P.traj_order != 2;
+    const bool cubic = P.traj_order != 2;
     if (cubic && P.n_iters != 2) return false;
-    if (!staged || cubic)
-        return P.nx >= kTI && (P.nz <= 96 ? lanes >= (shallow ? 0.75 : 0.875) : P.nx >= 96 && lanes >= 0.96);
+    if (!staged || cubic) return P.nx >= kTI && (P.nz <= 96 ? lanes >= 0.875 : P.nx >= 96 && lanes >= 0.96);
     const long long blocks = 3LL * tiles * ((P.ny + kTJ - 1) / kTJ) * ((P.nz + kTK - 1) / kTK);
-    return lanes >= (shallow ? 0.65 : 0.75) && (P.nx >= kTI || blocks <= 148 * Box<6>::min_blocks);
+    return lanes >= 0.75 && (P.nx >= kTI || blocks <= 148 * Box<6>::min_blocks);
 }
 
 size_t tma_padded_elems(const SlcParams &P, int comp)

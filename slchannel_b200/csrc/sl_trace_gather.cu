@@ -39,8 +39,9 @@ constexpr int kThreads = 256;
 // MODE 0: one foot of depth dt on field fn (SLAdvector.advect).
 // MODE 1: BDF1 predictor ubar + dt R(fn)            (solver.py:760-771).
 // MODE 2: BDF2 predictor 4/3 ubar - 1/3 ubarbar + (2/3)dt Rh (solver.py:846-903).
-// Launch geometry of k_sl: a block is kTileK consecutive z arrival points
-// (one warp each 32) x kTileJ y-rows at one x index; grid (z tiles, y tiles, nx).
+// Launch geometry: a block is kTileK consecutive z arrival points (one warp
+// each 32) x kTileJ y-rows at one x index; grid (z tiles, y tiles, nx).  k_sl
+// takes its tile as an argument (tile_log2).
 #ifndef SLC_SL_TILE_K
 #define SLC_SL_TILE_K 64
 #endif
@@ -99,10 +100,10 @@ template <int C, int O, int MODE, int TO>
 __global__ void __launch_bounds__(kThreads, O == 4 ? SLC_SL_O4_MIN_BLOCKS : SLC_SL_MIN_BLOCKS) k_sl(const __grid_constant__ SlcParams P, const __grid_constant__ Vel3 M, const double *__restrict__ fn,
                                                     const double *__restrict__ fnm1, double dt,
                                                     double *__restrict__ out,
-                                                    unsigned long long *nclamp)
+                                                    unsigned long long *nclamp, int tkl)
 {
-    const int k = blockIdx.x * kTileK + (threadIdx.x % kTileK);
-    const int j = blockIdx.y * kTileJ + (threadIdx.x / kTileK);
+    const int k = (blockIdx.x << tkl) + (threadIdx.x & ((1 << tkl) - 1));
+    const int j = blockIdx.y * (kThreads >> tkl) + (threadIdx.x >> tkl);
     const int i = blockIdx.z;
     overlap_begin();
     unsigned ncl = 0;
@@ -363,15 +364,27 @@ __global__ void k_lincomb_ens(const EnsInst *__restrict__ ins, const EnsItem *__
     }
 }
 
+// k_sl's tile along z, as a power of two: 64 levels, or 32 where 64 would leave
+// the last tile's second warp of every row without a point (steps: 97x75x81
+// tricubic trajectories 1353 -> 1220 us, 64x64x24 order 4 140 -> 130, 128x128x96
+// order 4 703 -> 662).
+int tile_log2(int levels) { return ((levels + 31) / 32) & 1 ? 5 : 6; }
+dim3 tile_grid(const SlcParams &P, int levels, int tkl)
+{
+    const int tk = 1 << tkl, tj = kThreads >> tkl;
+    return dim3((levels + tk - 1) / tk, (P.ny + tj - 1) / tj, P.nx);
+}
+
 template <int O, int MODE, int TO>
 void launch_sl_tt(const SlcParams &P, const Vel3 &M, Tri fn, Tri fnm1, double dt, TriMut out,
                   unsigned long long *ncl, cudaStream_t s)
 {
-    const dim3 gc((P.nz + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
-    const dim3 gw((P.nz - 1 + kTileK - 1) / kTileK, (P.ny + kTileJ - 1) / kTileJ, P.nx);
-    launch_chained(k_sl<0, O, MODE, TO>, gc, kThreads, 0, s, false, P, M, fn.u, fnm1.u, dt, out.u, ncl);
-    launch_chained(k_sl<1, O, MODE, TO>, gc, kThreads, 0, s, true, P, M, fn.v, fnm1.v, dt, out.v, ncl);
-    if (P.nz > 1) launch_chained(k_sl<2, O, MODE, TO>, gw, kThreads, 0, s, true, P, M, fn.w, fnm1.w, dt, out.w, ncl);
+    const int tc = tile_log2(P.nz), tw = tile_log2(P.nz - 1);
+    const dim3 gc = tile_grid(P, P.nz, tc), gw = tile_grid(P, P.nz - 1, tw);
+    launch_chained(k_sl<0, O, MODE, TO>, gc, kThreads, 0, s, false, P, M, fn.u, fnm1.u, dt, out.u, ncl, tc);
+    launch_chained(k_sl<1, O, MODE, TO>, gc, kThreads, 0, s, true, P, M, fn.v, fnm1.v, dt, out.v, ncl, tc);
+    if (P.nz > 1)
+        launch_chained(k_sl<2, O, MODE, TO>, gw, kThreads, 0, s, true, P, M, fn.w, fnm1.w, dt, out.w, ncl, tw);
     count_launches(P.nz > 1 ? 3 : 2);
 }
 

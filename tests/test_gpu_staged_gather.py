@@ -123,3 +123,15 @@ def test_staged_equals_l1_other_trajectories(n3, order, traj, iters):
         for c, x, y in zip("uvw", a, b):
             assert torch.isfinite(x).all() and torch.equal(x, y), (c, dt)
         assert na == nb
+
+
+@pytest.mark.parametrize("nz", [31, 32, 33, 63, 64, 65, 96, 97, 129])
+@pytest.mark.parametrize("order", [6, 4])
+def test_staged_equals_l1_at_tile_edges(nz, order):
+    """k_sl's 64- and 32-level tiles and the boxes' four levels against each other
+    around the tiles' ends (w has one level fewer)."""
+    f = _flow((32, 10, nz), 0.03, 0.1, order)
+    (a, na), (b, nb) = _both(f, 0.03)[0]
+    for c, x, y in zip("uvw", a, b):
+        assert float(x.abs().max()) > 0.0 and torch.equal(x, y), c
+    assert na == nb
